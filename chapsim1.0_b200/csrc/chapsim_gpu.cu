@@ -493,10 +493,12 @@ int configure_momentum(chapsim_ctx* ctx) {
     ctx->rb_nw = 0;
     DISPATCH_S(g.L / 32, ctx->rb_nw = rb_warps<R>(g.L, bulk_smem_limit(k_rhs_xsweep_bulk<S, R>)));
     if (ctx->rb_nw > 0) DISPATCH_S(g.L / 32, CK(set_smem(k_rhs_xsweep_bulk<S, R>, rb_smem<R>(g.L, ctx->rb_nw))));
-    DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 32, 1>, smem_z<R>(g, 32))));
-    DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 16, 1>, smem_z<R>(g, 16))));
-    DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 32, 2>, smem_z<R>(g, 32))));
-    DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 16, 2>, smem_z<R>(g, 16))));
+    if constexpr (sizeof(R) == 4) {
+        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 32, 1>, smem_z<R>(g, 32))));
+        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 16, 1>, smem_z<R>(g, 16))));
+        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 32, 2>, smem_z<R>(g, 32))));
+        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 16, 2>, smem_z<R>(g, 16))));
+    }
     DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, R, 1>, smem_y<R>(g))));
     DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, R, 2>, smem_y<R>(g))));
     DISPATCH_S(g.L / 32, CK(set_smem(k_xsweep<S, R>, smem_xs<R>(g))));
@@ -524,8 +526,9 @@ int configure_momentum(chapsim_ctx* ctx) {
 
 int configure_kernels(chapsim_ctx* ctx) {
     const Geo& g = ctx->g;
-    // z-sweep tiles before any tuning: 16 lines where 32-line FP64 tiles leave one block per SM
-    ctx->zs_tw = ctx->prec != CHAPSIM_PREC_MIXED && g.N / 32 >= 6 ? 16 : 32;
+    // z-sweep tiles before any tuning: FP64 in 16-line blocks (never slower than 32-line ones: 3.8 against 4.1 us
+    // at 64^3, 16.7 against 20.1 at 128^3, 323 against 343 us at 384 x 256 x 384)
+    ctx->zs_tw = ctx->prec != CHAPSIM_PREC_MIXED ? 16 : 32;
     int rc = ctx->prec == CHAPSIM_PREC_MIXED ? configure_momentum<float>(ctx) : configure_momentum<double>(ctx);
     if (rc) return rc;
     // the FP64 spectral stage serves the standalone Poisson solve and the main domain in every precision
@@ -673,14 +676,23 @@ void launch_pressure(chapsim_ctx* ctx, const StepFields<R>& f, int ns) {
     ctx->launches += 5;
 }
 
-// cyclic z sweep, persistent: as many blocks as fit at once (two per SM where the two tile
-// buffers allow); tiles of ctx->zs_tw lines
-template <typename R>
-void launch_zsweep(chapsim_ctx* ctx, const StepFields<R>& f, const R* fac) {
+// Cyclic z sweep.  FP64: the register form, tiles of ctx->zs_tw lines.  FP32: persistent, as many
+// blocks as fit at once (two per SM where the two tile buffers allow).
+void launch_zsweep(chapsim_ctx* ctx, const StepFields<double>& f, const double* fac) {
+    const Geo& g = ctx->g;
+    const int nz = (g.L / ctx->zs_tw) * (3 * g.M - 1);
+    if (ctx->zs_tw == 16) {
+        DISPATCH_SEG(g.N, (launch_pdl(ctx->pdl, k_zsweep_reg<NSEG, SR, 16>, nz, 16 * NSEG, 0, ctx->stream, g, f.RHS, fac)));
+    } else {
+        DISPATCH_SEG(g.N, (launch_pdl(ctx->pdl, k_zsweep_reg<NSEG, SR, 32>, nz, 32 * NSEG, 0, ctx->stream, g, f.RHS, fac)));
+    }
+}
+void launch_zsweep(chapsim_ctx* ctx, const StepFields<float>& f, const float* fac) {
+    using R = float;
     const Geo& g = ctx->g;
     const int tw = ctx->zs_tw;
     const size_t sz = smem_z<R>(g, tw);
-    const int zb_want = sizeof(R) == 4 && g.N / 32 <= 4 ? 3 : 2;  // zsweep_blocks<R, S>
+    const int zb_want = g.N / 32 <= 4 ? 3 : 2;  // zsweep_blocks<R, S>
     const int zb = sz * zb_want <= 226 * 1024 ? zb_want : (sz <= 113 * 1024 ? 2 : 1);
     const int nz = std::min((g.L / tw) * (3 * g.M - 1), zb * ctx->nsm);
     if (tw == 16 && ctx->zs_il == 2) {
@@ -721,7 +733,7 @@ void launch_substep_t(chapsim_ctx* ctx, int ns, bool factors) {
     }
     launch_rhs_x<R>(ctx, f, fac, ns);
     prof_mark(ctx);
-    launch_zsweep<R>(ctx, f, fac);
+    launch_zsweep(ctx, f, fac);
     prof_mark(ctx);
     launch_ysweep<R>(ctx, f, fac, ns);
     prof_mark(ctx);
@@ -2856,15 +2868,19 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
     if (ctx->domain == 1) {
         const bool mixed = ctx->prec == CHAPSIM_PREC_MIXED;
         for (int v = 0; v < 4; ++v) {
+            if (!mixed && v >= 2) {  // the FP64 sweep has no tile layout
+                tz[v] = tz[v & 1];
+                continue;
+            }
             ctx->zs_tw = (v & 1) ? 16 : 32;
             ctx->zs_il = (v & 2) ? 2 : 1;
             auto one = [&]() {
                 if (mixed) {
                     StepFields<float> f = step_fields<float>(ctx);
-                    launch_zsweep<float>(ctx, f, f.fac + 5 * FAC_SET);
+                    launch_zsweep(ctx, f, f.fac + 5 * FAC_SET);
                 } else {
                     StepFields<double> f = step_fields<double>(ctx);
-                    launch_zsweep<double>(ctx, f, f.fac + 5 * FAC_SET);
+                    launch_zsweep(ctx, f, f.fac + 5 * FAC_SET);
                 }
             };
             one();
@@ -2875,7 +2891,7 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
             CK(cudaEventElapsedTime(&tz[v], e0, e1));
             tz[v] /= reps;
         }
-        ctx->launches += 4 * (1 + reps);
+        ctx->launches += (mixed ? 4 : 2) * (1 + reps);
         CK(cudaGetLastError());
         int bz = 0;
         for (int v = 1; v < 4; ++v)

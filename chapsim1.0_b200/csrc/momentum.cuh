@@ -92,6 +92,21 @@ struct YCoef {  // MOMFA3_Y_tg rows: (-F*AMVR, 1 - F*ACVR, -F*APVR), row r = j-1
     __device__ __forceinline__ double C(int r) const { return -f * ap[r + 1]; }
 };
 
+// Segments of a line in the register sweeps: n = segments x rows, at most 24 rows per thread.
+__host__ __device__ constexpr int seg_rows(int n) { return n == 384 ? 24 : n == 256 ? 16 : n == 192 || n == 96 ? 12 : 8; }
+// Host dispatch on the line length: defines constexpr NSEG, SR for KERNEL_CALL.
+#define DISPATCH_SEG(n_, KERNEL_CALL)                                                    \
+    switch (n_) {                                                                       \
+        case 32: { constexpr int NSEG = 4, SR = 8; KERNEL_CALL; } break;                \
+        case 64: { constexpr int NSEG = 8, SR = 8; KERNEL_CALL; } break;                \
+        case 96: { constexpr int NSEG = 8, SR = 12; KERNEL_CALL; } break;               \
+        case 128: { constexpr int NSEG = 16, SR = 8; KERNEL_CALL; } break;              \
+        case 192: { constexpr int NSEG = 16, SR = 12; KERNEL_CALL; } break;             \
+        case 256: { constexpr int NSEG = 16, SR = 16; KERNEL_CALL; } break;             \
+        case 384: { constexpr int NSEG = 16, SR = 24; KERNEL_CALL; } break;             \
+        default: break;                                                                 \
+    }
+
 template <bool CYC, class C, typename T>
 __device__ void factor_dispatch(int S, const C& cf, int lane, T* fac) {
     switch (S) {
@@ -106,9 +121,36 @@ __device__ void factor_dispatch(int S, const C& cf, int lane, T* fac) {
     }
 }
 
+// Table of the FP64 z sweep (k_zsweep_reg).  The cyclic system with rows (a, 1 - 2a, a), a <= 0, factors
+// into c (1 - rho E^-1)(1 - rho E) with c = (1 + 2|a| + sqrt(1 + 4|a|)) / 2 and rho = |a| / c < 1 (E the
+// shift by one row), i.e. two first-order recurrences.  f[0] = 1/c, f[1] = 1/(1 - rho^n), f[2 + k] =
+// rho^k for k = 0..sr (sr rows per segment).
+#define ZT_POW 2
+__device__ __forceinline__ void zsweep_table(double a, int n, int sr, int lane, double* __restrict__ f) {
+    const double m = -a;
+    const double c = (1.0 + 2.0 * m + sqrt(1.0 + 4.0 * m)) * 0.5;
+    const double rho = m / c;
+    double p = 1.0, pn = 1.0;
+    for (int k = 0; k < n; ++k) {
+        pn *= rho;
+        if (k < lane) p *= rho;
+    }
+    if (lane <= sr) f[ZT_POW + lane] = p;
+    if (lane == 0) {
+        f[0] = 1.0 / c;
+        f[1] = 1.0 / (1.0 - pn);
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ void factor_set(const Geo& g, double dt, int ns, int set, T* f, int lane) {
     const double facoe = 0.5 * g.talp[ns] * dt * g.cvisc * 1.0 / 1.0;
+    if constexpr (sizeof(T) == 8) {
+        if (set == FSET_Z) {
+            zsweep_table(1.0 * (-facoe * g.dzqi), g.N, seg_rows(g.N), lane, f);  // MOMFA2_Z_tg :133-155
+            return;
+        }
+    }
     if (set == FSET_X) {
         ConstCoef cf;
         cf.a = -facoe * g.dxqi;  // MOMFA1_X_tg :72-78
@@ -537,6 +579,63 @@ __global__ void __launch_bounds__(SWEEP_NT, (zsweep_blocks<R, S>())) k_zsweep(Ge
         b ^= 1;
     }
     cp_async_wait_all();
+}
+
+// ---------------------------------------------------------------------------
+// FP64 cyclic z sweep in registers.  A block solves TI consecutive x lines of one (component, j): thread
+// (il, seg) owns the SR consecutive z rows of segment seg of line il, so every global access is a
+// row piece of TI doubles and nothing is staged or transposed.  The two recurrences of zsweep_table
+// run along the segment in registers; the segments' carries go through NSEG x TI doubles of shared
+// memory, where each thread sums the preceding (following) segments' totals around the ring by Horner's
+// rule in rho^SR and closes the ring with 1/(1 - rho^n).
+// All SR loads of a thread are independent and in flight together, and the factors are SR + 3 numbers
+// read by broadcast; the warp-per-line form (k_zsweep, still the FP32 one, whose results are kept to
+// the bit) loads 5 S + 20 factors per lane and line and moves each element four times through shared
+// memory.  Bound by HBM: 0.584 -> 0.323 ms per launch at 384 x 256 x 384 (0.47 -> 0.86 of the measured copy
+// bandwidth), 28.1 -> 16.7 us at 128^3.
+// Threads per SM the register budget is sized for (no spills): 512 at 24 rows, 768 at 12 and 16, 1024 at 8.
+template <int SR> __host__ __device__ constexpr int zr_minb(int nt) { return (SR > 16 ? 512 : SR > 8 ? 768 : 1024) / nt > 1 ? (SR > 16 ? 512 : SR > 8 ? 768 : 1024) / nt : 1; }
+template <int NSEG, int SR, int TI>
+__global__ void __launch_bounds__(TI * NSEG, zr_minb<SR>(TI * NSEG)) k_zsweep_reg(Geo g, double* __restrict__ RHS, const double* __restrict__ fac) {
+    pdl_wait();
+    static_assert((NSEG & (NSEG - 1)) == 0, "the ring of segments is indexed by a mask");
+    __shared__ double sT[NSEG][TI], sZ[NSEG][TI], spw[SR + 1];
+    const int M = g.M, nx = g.L / TI;
+    const int il = threadIdx.x % TI, seg = threadIdx.x / TI;
+    const int t = blockIdx.x;
+    int comp, j;  // tiles of v at j = 1 are skipped (MOMFA2_Z_tg starts at N2I = 2 for v)
+    if (t < nx * M) { comp = 0; j = 1 + t / nx; }
+    else if (t < nx * (2 * M - 1)) { comp = 1; j = 2 + (t - nx * M) / nx; }
+    else { comp = 2; j = 1 + (t - nx * (2 * M - 1)) / nx; }
+    const long long ks = g.PI_;
+    double* R = RHS + comp * g.FI + iidx(g, TI * (t % nx) + il, j, seg * SR);
+    double d[SR];
+#pragma unroll
+    for (int k = 0; k < SR; ++k) d[k] = R[ks * k];
+    const double* fz = fac + FSET_Z * FAC_SET;
+    if (threadIdx.x <= SR) spw[threadIdx.x] = fz[ZT_POW + threadIdx.x];
+    const double ic = fz[0], ring = fz[1], rho = fz[ZT_POW + 1], q = fz[ZT_POW + SR];
+    d[0] *= ic;
+#pragma unroll
+    for (int k = 1; k < SR; ++k) d[k] = fma(rho, d[k - 1], d[k] * ic);
+    sT[seg][il] = d[SR - 1];
+    __syncthreads();
+    double c = sT[seg][il];
+#pragma unroll 4
+    for (int m = NSEG - 1; m >= 1; --m) c = fma(c, q, sT[(seg - m) & (NSEG - 1)][il]);
+    c *= ring;
+#pragma unroll
+    for (int k = 0; k < SR; ++k) d[k] = fma(spw[k + 1], c, d[k]);
+#pragma unroll
+    for (int k = SR - 2; k >= 0; --k) d[k] = fma(rho, d[k + 1], d[k]);
+    sZ[seg][il] = d[0];
+    __syncthreads();
+    c = sZ[seg][il];
+#pragma unroll 4
+    for (int m = NSEG - 1; m >= 1; --m) c = fma(c, q, sZ[(seg + m) & (NSEG - 1)][il]);
+    c *= ring;
+#pragma unroll
+    for (int k = 0; k < SR; ++k) R[ks * k] = fma(spw[SR - k], c, d[k]);
 }
 
 // ---------------------------------------------------------------------------
