@@ -164,8 +164,8 @@ struct chapsim_ctx {
                                   // fused form, 16-byte loads (rhs_pv) (chapsim_autotune)
     int plane_kind = 0;           // 0: chained x/z transforms, 1: fused plane transforms k_div_fft2/k_fft2_inv (chapsim_autotune)
     int zs_tw = 32;               // lines per tile of the z sweep, 32 or 16 (chapsim_autotune)
-    int zs_il = 1;                // z-sweep tile layout: 1 line-contiguous, 2 lines interleaved in pairs (chapsim_autotune)
-    int ys_il = 1;                // the same for the y sweep (chapsim_autotune)
+    int zs_il = 1;                // FP32 z-sweep tile layout: 1 line-contiguous, 2 lines interleaved in pairs (chapsim_autotune)
+    int ys_il = 1;                // the same for the FP32 y sweep (chapsim_autotune)
     bool fz_pipe = false;         // persistent double-buffered z transforms (chapsim_autotune)
     bool fz_prefetch = false;     // one-tile z transforms request the tile one wave ahead into L2 (chapsim_autotune)
     bool p2c = false;             // the fused plane transforms run as a thread-block cluster (k_div_fft2c/k_fft2c_inv)
@@ -498,9 +498,9 @@ int configure_momentum(chapsim_ctx* ctx) {
         DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 16, 1>, smem_z<R>(g, 16))));
         DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 32, 2>, smem_z<R>(g, 32))));
         DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 16, 2>, smem_z<R>(g, 16))));
+        DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, R, 1>, smem_y<R>(g))));
+        DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, R, 2>, smem_y<R>(g))));
     }
-    DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, R, 1>, smem_y<R>(g))));
-    DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, R, 2>, smem_y<R>(g))));
     DISPATCH_S(g.L / 32, CK(set_smem(k_xsweep<S, R>, smem_xs<R>(g))));
     CK(set_smem(k_rhs_point<R>, smem_rt<R>()));
     using C = SpecT<R>;
@@ -706,9 +706,16 @@ void launch_zsweep(chapsim_ctx* ctx, const StepFields<float>& f, const float* fa
     }
 }
 
-// y sweep + update, the tile layout ctx->ys_il (chapsim_autotune bit 11)
-template <typename R>
-void launch_ysweep(chapsim_ctx* ctx, const StepFields<R>& f, const R* fac, int ns) {
+// y sweep + update.  FP64: the register form, 16 lines per block; FP32: the tile layout ctx->ys_il
+// (chapsim_autotune bit 11).
+void launch_ysweep(chapsim_ctx* ctx, const StepFields<double>& f, const double* fac, int ns) {
+    const Geo& g = ctx->g;
+    dim3 gry(g.L / 16, g.N, 2);  // layer 0: u then v, layer 1: w
+    DISPATCH_SEG(g.M, (launch_pdl(ctx->pdl, k_ysweep_reg<NSEG * SR / yseg_rows(NSEG * SR), yseg_rows(NSEG * SR), 16>, gry,
+                                  16 * (NSEG * SR / yseg_rows(NSEG * SR)), 0, ctx->stream, g, f.Q, f.RHS, ctx->st, fac, ns)));
+}
+void launch_ysweep(chapsim_ctx* ctx, const StepFields<float>& f, const float* fac, int ns) {
+    using R = float;
     const Geo& g = ctx->g;
     dim3 gry(g.L / 32, g.N, 2);  // layer 0: u then v, layer 1: w
     if (ctx->ys_il == 2) {
@@ -735,7 +742,7 @@ void launch_substep_t(chapsim_ctx* ctx, int ns, bool factors) {
     prof_mark(ctx);
     launch_zsweep(ctx, f, fac);
     prof_mark(ctx);
-    launch_ysweep<R>(ctx, f, fac, ns);
+    launch_ysweep(ctx, f, fac, ns);
     prof_mark(ctx);
     launch_pressure<R>(ctx, f, ns);
     const long long tot = (long long)g.L * g.M * g.N / V16<R>::W;  // one thread per 16-byte group of an x line
@@ -2911,14 +2918,18 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
         void* q0 = mixed ? (void*)ctx->Qf : (void*)ctx->Q;
         CK(cudaMemcpyAsync(qsave, q0, qb, cudaMemcpyDeviceToDevice, s));
         for (int v = 0; v < 2; ++v) {
+            if (!mixed && v == 1) {  // the FP64 sweep has no tile layout
+                ty[1] = ty[0];
+                continue;
+            }
             ctx->ys_il = v + 1;
             auto one = [&]() {
                 if (mixed) {
                     StepFields<float> f = step_fields<float>(ctx);
-                    launch_ysweep<float>(ctx, f, f.fac + 5 * FAC_SET, 1);
+                    launch_ysweep(ctx, f, f.fac + 5 * FAC_SET, 1);
                 } else {
                     StepFields<double> f = step_fields<double>(ctx);
-                    launch_ysweep<double>(ctx, f, f.fac + 5 * FAC_SET, 1);
+                    launch_ysweep(ctx, f, f.fac + 5 * FAC_SET, 1);
                 }
             };
             one();
@@ -2929,7 +2940,7 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
             CK(cudaEventElapsedTime(&ty[v], e0, e1));
             ty[v] /= reps;
         }
-        ctx->launches += 2 * (1 + reps);
+        ctx->launches += (mixed ? 2 : 1) * (1 + reps);
         CK(cudaMemcpyAsync(q0, qsave, qb, cudaMemcpyDeviceToDevice, s));
         CK(cudaStreamSynchronize(s));
         cudaFree(qsave);

@@ -94,7 +94,8 @@ struct YCoef {  // MOMFA3_Y_tg rows: (-F*AMVR, 1 - F*ACVR, -F*APVR), row r = j-1
 
 // Segments of a line in the register sweeps: n = segments x rows, at most 24 rows per thread.
 __host__ __device__ constexpr int seg_rows(int n) { return n == 384 ? 24 : n == 256 ? 16 : n == 192 || n == 96 ? 12 : 8; }
-// Host dispatch on the line length: defines constexpr NSEG, SR for KERNEL_CALL.
+__host__ __device__ constexpr int yseg_rows(int n) { return n == 384 ? 16 : seg_rows(n); }  // y sweep: at most 16 rows
+// Host dispatch on the z-line length: defines constexpr NSEG, SR for KERNEL_CALL.
 #define DISPATCH_SEG(n_, KERNEL_CALL)                                                    \
     switch (n_) {                                                                       \
         case 32: { constexpr int NSEG = 4, SR = 8; KERNEL_CALL; } break;                \
@@ -142,12 +143,74 @@ __device__ __forceinline__ void zsweep_table(double a, int n, int sr, int lane, 
     }
 }
 
+// Table of the FP64 y sweep of one component (k_ysweep_reg): the LU recurrences of the sequential solve,
+//   g_j = PP_j r_j - (A_j PP_j) g_{j-1},   x_j = g_j - H_j x_{j+1},
+// PP_j = 1/(B_j - A_j H_{j-1}), H_j = C_j PP_j.  Row j (0-based): f[4 j] = PP_j, f[4 j + 1] = -A_j PP_j,
+// f[4 j + 2] = -H_j; then per segment of sr rows the products of f[4 j + 1] (at YT_SEG(n) + s) and of
+// f[4 j + 2] (at YT_SEG(n) + 32 + s).  One warp, S = n / 32 rows per lane: every lane runs its rows' pivot
+// chain from the H its neighbour last produced, until no lane's incoming H changes; that fixed point
+// is the sequential recurrence bit for bit, and as the chain forgets its start within a few rows
+// (H_j depends on H_{j-1} with a factor A_j C_j PP_j^2) a few rounds reach it, at most 32.
+#define YT_SEG(n) (4 * (n))
+template <int S, class Coef>
+__device__ __forceinline__ void ysweep_table(const Coef& cf, int sr, int lane, double* __restrict__ f) {
+    constexpr int n = 32 * S;
+    double pp[S], hh[S], hin = 0.0;
+    for (int round = 0; round < 33; ++round) {
+        double h = hin;
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            const int r = lane * S + k;
+            pp[k] = 1.0 / (cf.B(r) - (r == 0 ? 0.0 : cf.A(r)) * h);
+            hh[k] = h = r == n - 1 ? 0.0 : cf.C(r) * pp[k];
+        }
+        const double up = __shfl_up_sync(0xffffffffu, h, 1);
+        const double nh = lane == 0 ? 0.0 : up;
+        const bool moved = nh != hin;
+        hin = nh;
+        if (!__any_sync(0xffffffffu, moved)) break;
+    }
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+        const int r = lane * S + k;
+        f[4 * r] = pp[k];
+        f[4 * r + 1] = r == 0 ? 0.0 : -cf.A(r) * pp[k];
+        f[4 * r + 2] = -hh[k];
+        f[4 * r + 3] = 0.0;
+    }
+    __syncwarp();
+    if (lane < n / sr) {
+        double a = 1.0, h = 1.0;
+        for (int k = 0; k < sr; ++k) {
+            a *= f[4 * (lane * sr + k) + 1];
+            h *= f[4 * (lane * sr + k) + 2];
+        }
+        f[YT_SEG(n) + lane] = a;
+        f[YT_SEG(n) + 32 + lane] = h;
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ void factor_set(const Geo& g, double dt, int ns, int set, T* f, int lane) {
     const double facoe = 0.5 * g.talp[ns] * dt * g.cvisc * 1.0 / 1.0;
     if constexpr (sizeof(T) == 8) {
         if (set == FSET_Z) {
             zsweep_table(1.0 * (-facoe * g.dzqi), g.N, seg_rows(g.N), lane, f);  // MOMFA2_Z_tg :133-155
+            return;
+        }
+        if (set >= FSET_Y) {  // MOMFA3_Y_tg :172-238
+            const int comp = set - FSET_Y, sr = yseg_rows(g.M);
+            const YCoef cf{g.amvr + comp * (g.M + 2), g.acvr + comp * (g.M + 2), g.apvr + comp * (g.M + 2), facoe};
+            switch (g.M / 32) {
+                case 1: ysweep_table<1>(cf, sr, lane, f); break;
+                case 2: ysweep_table<2>(cf, sr, lane, f); break;
+                case 3: ysweep_table<3>(cf, sr, lane, f); break;
+                case 4: ysweep_table<4>(cf, sr, lane, f); break;
+                case 6: ysweep_table<6>(cf, sr, lane, f); break;
+                case 8: ysweep_table<8>(cf, sr, lane, f); break;
+                case 12: ysweep_table<12>(cf, sr, lane, f); break;
+                default: break;
+            }
             return;
         }
     }
@@ -738,6 +801,90 @@ __global__ void __launch_bounds__(SWEEP_NT, (S >= 6 ? 2 : (sizeof(R) == 4 ? 4 : 
             }
         }
         __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// FP64 y sweep + Q update in registers: the thread layout of k_zsweep_reg (thread (il, seg) owns SR
+// consecutive y rows of x line il at fixed k), the recurrences of ysweep_table, whose factors are the
+// same for every line and are read by broadcast (24 bytes per row), and the segments' carries summed
+// by Horner's rule over the preceding (following) segments.  The multipliers of both recurrences are
+// loaded while the right-hand sides are on their way (read inside the chains, their L1 latency set the
+// kernel's pace: 0.575 ms per launch at 384 x 256 x 384), and the Q rows when the forward multipliers'
+// registers are free.  0.556 -> 0.516 ms there (0.75 -> 0.81 of the measured copy bandwidth), 40.7 ->
+// 33.4 us at 128^3.  Components and grid layers as in k_ysweep.
+template <int SR> __host__ __device__ constexpr int yr_minb(int nt) { return (SR > 8 ? 512 : 768) / nt > 1 ? (SR > 8 ? 512 : 768) / nt : 1; }
+template <int NSEG, int SR, int TI>
+__global__ void __launch_bounds__(TI * NSEG, yr_minb<SR>(TI * NSEG)) k_ysweep_reg(Geo g, double* __restrict__ Q, const double* __restrict__ RHS,
+                                                                              const DevState* __restrict__ st,
+                                                                              const double* __restrict__ fac, int ns) {
+    pdl_wait();
+    __shared__ double sT[NSEG][TI], sZ[NSEG][TI], sdu[TI], sseg[64];
+    const int il = threadIdx.x % TI, seg = threadIdx.x / TI;
+    const int i = blockIdx.x * TI + il, k = blockIdx.y;
+    const long long js = g.L;  // stride between y rows (interior and padded fields alike)
+    // DPGRNS (RHS_CvLpGpS_tg :163-199)
+    double dpg = 0.0;
+    if (g.iflowdriven == 1) dpg = st->bulksum / g.volm;
+    else if (g.iflowdriven == 2) dpg = -0.5 * g.cf_given * (g.talp[ns] * st->dt / 1.0);
+    const int comp_lo = blockIdx.z == 0 ? 0 : 2, comp_hi = blockIdx.z == 0 ? 2 : 3;
+#pragma unroll 1
+    for (int comp = comp_lo; comp < comp_hi; ++comp) {
+        const double* R = RHS + comp * g.FI + iidx(g, i, 1 + seg * SR, k);
+        double* Qc = Q + comp * g.FS + pidx(g, i, 1 + seg * SR, k);
+        double d[SR], al[SR], et[SR];
+#pragma unroll
+        for (int r = 0; r < SR; ++r) d[r] = R[js * r];
+        const double* fy = fac + (FSET_Y + comp) * FAC_SET;
+        const double2* fr = reinterpret_cast<const double2*>(fy) + 2 * seg * SR;
+        for (int t = threadIdx.x; t < 64; t += TI * NSEG) sseg[t] = fy[YT_SEG(NSEG * SR) + t];
+        if (comp == 0) {
+#pragma unroll
+            for (int r = 0; r < SR; ++r) d[r] -= dpg;
+        } else if (comp == 1 && seg == 0) {
+            d[0] = g.fix_v_wall_row ? 0.0 : sdu[il];  // row 1 of v: see the quirk note above
+        }
+#pragma unroll
+        for (int r = 0; r < SR; ++r) {
+            const double2 w = fr[2 * r];
+            al[r] = w.y;
+            et[r] = fr[2 * r + 1].x;
+            d[r] *= w.x;
+        }
+#pragma unroll
+        for (int r = 1; r < SR; ++r) d[r] = fma(al[r], d[r - 1], d[r]);
+        sT[seg][il] = d[SR - 1];
+        __syncthreads();
+        double c = 0.0;
+#pragma unroll 4
+        for (int m = 0; m < NSEG - 1; ++m)
+            if (m < seg) c = fma(c, sseg[m], sT[m][il]);
+#pragma unroll
+        for (int r = 0; r < SR; ++r) {
+            c *= al[r];
+            d[r] += c;
+        }
+        double q[SR];
+#pragma unroll
+        for (int r = 0; r < SR; ++r) q[r] = Qc[js * r];
+#pragma unroll
+        for (int r = SR - 2; r >= 0; --r) d[r] = fma(et[r], d[r + 1], d[r]);
+        sZ[seg][il] = d[0];
+        __syncthreads();
+        c = 0.0;
+#pragma unroll 4
+        for (int m = NSEG - 1; m >= 1; --m)
+            if (m > seg) c = fma(c, sseg[32 + m], sZ[m][il]);
+#pragma unroll
+        for (int r = SR - 1; r >= 0; --r) {
+            c *= et[r];
+            d[r] += c;
+        }
+        if (comp == 0 && seg == 0) sdu[il] = d[0];  // read by v's segment 0 only: the same thread
+#pragma unroll
+        for (int r = 0; r < SR; ++r)
+            if (comp != 1 || r > 0 || seg > 0) Qc[js * r] = d[r] + q[r];
+        __syncthreads();  // the carries and segment products are rewritten by the next component
     }
 }
 

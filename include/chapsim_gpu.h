@@ -517,7 +517,9 @@ int chapsim_dump_write(chapsim_ctx_t* ctx, const char* path_prefix, int32_t iter
  *          one (periodic channel only; timed as a third pressure-stage form);
  *   bit 10: z-sweep tile layout (periodic channel only), 0 = each x line
  *          contiguous in shared memory, 1 = lines interleaved in pairs (one
- *          copy instruction per two points);
+ *          copy instruction per two points); in FP64, whose sweeps hold
+ *          their lines in registers, bits 10 and 11 are kept but have no
+ *          effect;
  *   bit 11: the same for the y sweep (Q is restored after its trials);
  *   bit 12: with the chained transforms, each z-transform block also
  *          requests into L2 the tile of the block one wave later (timed as a
