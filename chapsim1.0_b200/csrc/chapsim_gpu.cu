@@ -544,12 +544,8 @@ int configure_kernels(chapsim_ctx* ctx) {
     DISPATCH_FFT(g.N, CK(set_smem(k_fftz<-1, FN1, FN2, double2>, smem_fz(g))));
     DISPATCH_FFT(g.N, CK(set_smem(k_fftz<+1, FN1, FN2, double2>, smem_fz(g))));
     if (ctx->domain == 2 && ctx->ivis) {
-        DISPATCH_S(g.L / 32, CK(set_smem(k_io_cn_xsweep<S, double>, smem_cn(g.L))));
-        DISPATCH_S(g.N / 32, CK(set_smem(k_io_cn_zsweep<S, double>, smem_cn(g.N))));
-        DISPATCH_S(g.M / 32, CK(set_smem(k_io_cn_ysweep<S, double>, smem_cn(g.M))));
-        DISPATCH_S(g.L / 32, CK(set_smem(k_io_cn_xsweep<S, float>, smem_cn(g.L))));
-        DISPATCH_S(g.N / 32, CK(set_smem(k_io_cn_zsweep<S, float>, smem_cn(g.N))));
-        DISPATCH_S(g.M / 32, CK(set_smem(k_io_cn_ysweep<S, float>, smem_cn(g.M))));
+        DISPATCH_S(g.L / 32, CK(set_smem(k_io_cn_xsweep<S * 32 / cn_w<double>(), double>, smem_cn_x<double>(g.L))));
+        DISPATCH_S(g.L / 32, CK(set_smem(k_io_cn_xsweep<S * 32 / cn_w<float>(), float>, smem_cn_x<float>(g.L))));
     }
     return CHAPSIM_OK;
 }
@@ -901,12 +897,13 @@ void launch_io_substep_t(chapsim_ctx* ctx, int ns) {
         // VISCOUS_PAR_EXPLT_* + RHS_MOM_EXPLICIT_io, then MOMFA_io's sweeps for all components
         k_io_rhs<true, F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->part_rhs, ctx->st, ns);
         prof_mark(ctx);
-        dim3 gx((unsigned)((g.M * (long long)g.N + CN_LINES - 1) / CN_LINES), 3);
-        DISPATCH_S(g.L / 32, (k_io_cn_xsweep<S, F><<<gx, CN_NT, smem_cn(g.L), s>>>(g, f, ctx->st, ns)));
+        constexpr int XS = 32 / cn_w<F>();  // segment length over DISPATCH_S's n / 32
+        dim3 gx((unsigned)((g.M * (long long)g.N + cn_xlines<F>() - 1) / cn_xlines<F>()), 3);
+        DISPATCH_S(g.L / 32, (k_io_cn_xsweep<S * XS, F><<<gx, CN_XNT, smem_cn_x<F>(g.L), s>>>(g, f, ctx->st, ns)));
         prof_mark(ctx);
-        dim3 gz(g.L / CN_LINES, g.M, 3), gy(g.L / CN_LINES, g.N, 3);
-        DISPATCH_S(g.N / 32, (k_io_cn_zsweep<S, F><<<gz, CN_NT, smem_cn(g.N), s>>>(g, f, ctx->st, ns)));
-        DISPATCH_S(g.M / 32, (k_io_cn_ysweep<S, F><<<gy, CN_NT, smem_cn(g.M), s>>>(g, f, ctx->st, ns)));
+        dim3 gz(g.L / cn_ti<F>(), g.M, 3), gy(g.L / cn_ti<F>(), g.N, 3);
+        DISPATCH_S(g.N / 32, (k_io_cn_zsweep<S * XS, F><<<gz, CN_NT, 0, s>>>(g, f, ctx->st, ns)));
+        DISPATCH_S(g.M / 32, (k_io_cn_ysweep<S * XS, F><<<gy, CN_NT, 0, s>>>(g, f, ctx->st, ns)));
         prof_mark(ctx);
         ctx->launches += 1;
     }

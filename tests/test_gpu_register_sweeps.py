@@ -1,5 +1,6 @@
-"""The FP64 z and y sweeps in registers, at every line length and both tile
-widths, against the oracle's sequential line solves.
+"""The line sweeps in registers at every line length, against the oracle's
+sequential line solves: the FP64 z and y sweeps of the periodic channel (both
+tile widths) and the Crank-Nicolson sweeps of the main domain.
 
 REN = 2 makes the implicit operators stiff (|a| = F / dz^2 from 1 to 190 at
 these grids, where the recurrences' ratio rho approaches 1 and carries travel
@@ -46,3 +47,33 @@ def test_stiff_sweeps_match_oracle(shape):
         for i in range(3):
             e = float(np.abs(Qg[i] - Qo[i]).max() / np.abs(Qo[i]).max())
             assert e <= 1e-11, (force, i, e)
+
+
+@pytest.mark.parametrize("shape", [(32, 384, 64), (64, 32, 32), (96, 64, 96), (128, 96, 384), (192, 128, 128),
+                                   (256, 192, 192), (384, 256, 256)])
+def test_stiff_main_domain_sweeps_match_oracle(shape):
+    """Non-uniform density and viscosity (each row has its own coefficients), two steps at REN = 2."""
+    L, M, N = shape
+    HX, HZ, REN, DT = 2 * math.pi, math.pi, 2.0, 5e-3
+    s = channel_setup(L, M, N, HX, HZ, 2.0, REN)
+    G, PR = initial_field(s, 43, 0.1)
+    k, j, i = np.meshgrid(np.arange(N), np.arange(M + 2), np.arange(L), indexing="ij")
+    rho = 1.0 + 0.05 * np.sin(2 * np.pi * i / L) * np.cos(2 * np.pi * k / N) + 0.02 * np.cos(np.pi * j / (M + 2))
+    mu0 = 1.0 + 0.1 * np.cos(2 * np.pi * i / L + 0.3) * np.sin(np.pi * j / (M + 2))
+    mu = mu0 * (1.0 + 0.03 * np.sin(2 * np.pi * k / N + 0.7))
+    o = Oracle(L, M, N, HX, HZ, 2.0, REN, DT0=DT, DTMIN=1e-6, CFLGV=1e9, threads=8)
+    o.io_set_fields(G, PR, rho, mu0, mu)
+    o.io_set_vis_scheme(1)
+    o.set_dt(DT)
+    assert o.io_run_steps(2)[0] == 0
+    Go = o.io_get_fields()[0]
+    o.close()
+    c = gpu.ChannelIO(s, ivisscheme=gpu.VIS_IMPLICIT)
+    c.upload_io(G, PR, rho, mu0, mu)
+    c.set_dt(DT)
+    c.advance(2, DT, 1e-6, 1e9)
+    Gg = c.download_io()[0]
+    c.close()
+    for q in range(3):
+        e = float(np.abs(Gg[q] - Go[q]).max() / np.abs(Go[q]).max())
+        assert e <= 1e-11, (q, e)
