@@ -103,9 +103,7 @@ def heated_kernel_words(L, M):
         "k_eng_rhs": 10.0,                            # H, T, kappa, G x3, DH, RHS_E0 in; DH, RHS_E0 out
         "k_eng_props": 11.0, "k_mlp_infer": 11.0,     # DH, DENSITY, Viscousity in; 8 property fields out
         "k_eng_bc": 22.0 / M,                         # the two ghost planes
-        "k_drhodt": 7.0,                              # G x3, G0 x3 in; DrhoDt out
-        "k_io_props": 8.0,                            # DENSITY0, Viscousity0 in; D_STG x3, MU_STG x3 out
-        "k_g0_velocity": 12.0,                        # G, D_STG in; G0, Q out (x3 each)
+        "k_eng_state": 17.0,                          # G x3, div G0, DENSITY0, Viscousity0 in; DrhoDt, div G, D_STG x3, MU_STG x3, Q x3 out
         "k_io_rhs_cn": 20.0,                          # G, Q, MU_STG, EXPLT0 (x3), Viscousity, PR in; EXPLT0, RHS out
         "k_io_cn_xsweep": 12.0,                       # RHS x3 in/out; 2 coefficient fields per component
         "k_io_cn_zysweep": 27.0,                      # z: as x; y: coefficients, RHS in, G in/out

@@ -711,8 +711,8 @@ class ChannelIO(ChannelTG):
     def kernel_slots(self):
         mom = (["k_io_rhs_cn", "k_io_cn_xsweep", "k_io_cn_zysweep"] if self.ivisscheme
                else ["k_io_divu", "k_io_rhs", "k_io_massflux"])
-        eng = (["k_eng_rhs", "k_mlp_infer" if self.use_mlp else "k_eng_props", "k_eng_bc", "k_drhodt", "k_io_props",
-                "k_g0_velocity"] if self.thermal else [])
+        eng = (["k_eng_rhs", "k_mlp_infer" if self.use_mlp else "k_eng_props", "k_eng_bc", "k_eng_state", None,
+                None] if self.thermal else [])
         sub = eng + mom + ["k_io_div_fftx", "k_fftz_fwd", "k_ysolve", "k_fftz_inv", "k_fftx_inv", "k_io_correct"]
         return ["k_io_cfl", "k_dt"] + sub * 3
 

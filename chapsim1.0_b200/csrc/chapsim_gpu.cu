@@ -862,13 +862,11 @@ void launch_thermal_substep_t(chapsim_ctx* ctx, int ns) {
         k_eng_bc<false, F><<<prop_grid(ctx, plane), PROP_NT, 0, s>>>(ctx->tab, g, f, ctx->tf, ctx->tp, ctx->st);
     }
     prof_mark(ctx);
-    k_drhodt<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->tf, ns, ctx->domain == 3 ? ctx->xio_mpart : nullptr);
+    k_eng_state<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->tf, ns, ctx->domain == 3 ? ctx->xio_mpart : nullptr);
     prof_mark(ctx);
-    k_io_props<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f);
+    prof_mark(ctx);  // two slots stay empty
     prof_mark(ctx);
-    k_g0_velocity<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->tf.G0);
-    prof_mark(ctx);
-    ctx->launches += 6;
+    ctx->launches += 4;
 }
 
 void launch_io_step_start(chapsim_ctx* ctx) {
@@ -1350,7 +1348,7 @@ void chapsim_gpu_finalize(chapsim_ctx_t* ctx) {
     cudaFree(ctx->mlp_par); cudaFree(ctx->mlp_w2); cudaFree(ctx->mlp_xs); cudaFree(ctx->mlp_ys); cudaFree(ctx->mlp_dh);
     cudaFree(ctx->mlp_judge);
     cudaFree(ctx->DEN); cudaFree(ctx->tf.DH); cudaFree(ctx->tf.ENTH); cudaFree(ctx->tf.TEMP); cudaFree(ctx->tf.KAP);
-    cudaFree(ctx->tf.HCP); cudaFree(ctx->tf.RHSE0); cudaFree(ctx->tf.G0); cudaFree(ctx->tf.DRHO);
+    cudaFree(ctx->tf.HCP); cudaFree(ctx->tf.RHSE0); cudaFree(ctx->tf.DIVG0); cudaFree(ctx->tf.DRHO);
     cudaFree(ctx->Qf); cudaFree(ctx->PRf); cudaFree(ctx->H0f); cudaFree(ctx->RHSf); cudaFree(ctx->RHSLLf); cudaFree(ctx->facf);
     if (ctx->st_host) cudaFreeHost(ctx->st_host);
     if (ctx->dump_stream) cudaStreamSynchronize(ctx->dump_stream);
@@ -2359,8 +2357,7 @@ void thermal_start(chapsim_ctx* ctx, size_t fb) {
     else k_eng_bc<false, F><<<prop_grid(ctx, plane), PROP_NT, 0, s>>>(ctx->tab, g, f, ctx->tf, ctx->tp, ctx->st);
     cudaMemcpyAsync(ctx->io.RHO, ctx->DEN, fb, cudaMemcpyDeviceToDevice, s);
     cudaMemcpyAsync(ctx->io.MU0, ctx->io.MU, fb, cudaMemcpyDeviceToDevice, s);
-    if constexpr (sizeof(F) == 8) cudaMemcpyAsync(ctx->tf.G0, f.G, 3 * fb, cudaMemcpyDeviceToDevice, s);
-    else k_convert<double, float><<<4 * ctx->nsm, DG_NT, 0, s>>>(ctx->tf.G0, f.G, 3 * g.FS);
+    k_eng_divg0<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->tf);
     k_io_props<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f);
     k_io_velocity<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f);
     ctx->launches += 5;
@@ -2412,7 +2409,7 @@ extern "C" int chapsim_thermal_init(chapsim_ctx_t* ctx, const double* dh, double
             CK(cudaMalloc(a, fb));
             CK(cudaMemsetAsync(*a, 0, fb, s));
         }
-        CK(cudaMalloc(&ctx->tf.G0, 3 * fb));
+        CK(cudaMalloc(&ctx->tf.DIVG0, fb));
     }
     ctx->tp.wf_bot = qw_bot;
     ctx->tp.wf_top = -qw_top;

@@ -62,35 +62,46 @@ __device__ __forceinline__ double io_pgm(const IoFieldsT<F>& f, long long c, lon
 
 
 // ---------------------------------------------------------------------------
+// DENSITY_Staggered and MU_Staggered at one point; d1, d2, d3 receive the point's D_STG as stored
+template <typename F>
+__device__ __forceinline__ void io_props_point(const Geo& g, const IoFieldsT<F>& f, int i, int j, int k, F& d1, F& d2, F& d3) {
+    const int im = xmn(g, i), km = wrapm(k, g.N);
+    const long long c = pidx(g, i, j, k);
+    const double* R = f.RHO;
+    const double* U0 = f.MU0;
+    d1 = (F)((R[c] + R[pidx(g, im, j, k)]) * 0.5);
+    d3 = (F)((R[c] + R[pidx(g, i, j, km)]) * 0.5);
+    d2 = (F)(j >= 2 ? g.wff[j] * R[c] + g.wfb[j] * R[pidx(g, i, j - 1, k)] : R[pidx(g, i, 0, k)]);
+    F m1, m3;
+    if (j >= 2) {
+        m1 = (F)(((U0[c] + U0[pidx(g, im, j, k)]) * g.wff[j] + (U0[pidx(g, i, j - 1, k)] + U0[pidx(g, im, j - 1, k)]) * g.wfb[j]) * 0.5);
+        m3 = (F)(((U0[pidx(g, i, j, km)] + U0[c]) * g.wff[j] + (U0[pidx(g, i, j - 1, km)] + U0[pidx(g, i, j - 1, k)]) * g.wfb[j]) * 0.5);
+    } else {
+        m1 = m3 = (F)U0[pidx(g, i, 0, k)];
+    }
+    const F m2 = (F)((U0[c] + U0[pidx(g, im, j, k)] + U0[pidx(g, i, j, km)] + U0[pidx(g, im, j, km)]) * 0.5 * 0.5);
+    f.DST[c] = d1;
+    f.DST[c + g.FS] = d2;
+    f.DST[c + 2 * g.FS] = d3;
+    f.MST[c] = m1;
+    f.MST[c + g.FS] = m2;
+    f.MST[c + 2 * g.FS] = m3;
+    if (j == g.M) {
+        const long long ct = pidx(g, i, g.M + 1, k);
+        f.DST[ct + g.FS] = (F)R[ct];
+        f.MST[ct] = (F)U0[ct];
+        f.MST[ct + 2 * g.FS] = (F)U0[ct];
+    }
+}
+
 template <typename F>
 __global__ void __launch_bounds__(IO_NT) k_io_props(Geo g, IoFieldsT<F> f) {
-    const int M = g.M, N = g.N;
     const long long tot = io_points(g);
     for (long long t = (long long)blockIdx.x * IO_NT + threadIdx.x; t < tot; t += (long long)gridDim.x * IO_NT) {
         int i, j, k;
         io_decode(g, t, i, j, k);
-        const int im = xmn(g, i), km = wrapm(k, N);
-        const long long c = pidx(g, i, j, k);
-        const double* R = f.RHO;
-        const double* U0 = f.MU0;
-        f.DST[c] = (F)((R[c] + R[pidx(g, im, j, k)]) * 0.5);
-        f.DST[c + 2 * g.FS] = (F)((R[c] + R[pidx(g, i, j, km)]) * 0.5);
-        f.DST[c + g.FS] = (F)(j >= 2 ? g.wff[j] * R[c] + g.wfb[j] * R[pidx(g, i, j - 1, k)] : R[pidx(g, i, 0, k)]);
-        if (j >= 2) {
-            f.MST[c] = (F)(((U0[c] + U0[pidx(g, im, j, k)]) * g.wff[j] + (U0[pidx(g, i, j - 1, k)] + U0[pidx(g, im, j - 1, k)]) * g.wfb[j]) * 0.5);
-            f.MST[c + 2 * g.FS] = (F)(((U0[pidx(g, i, j, km)] + U0[c]) * g.wff[j] +
-                                   (U0[pidx(g, i, j - 1, km)] + U0[pidx(g, i, j - 1, k)]) * g.wfb[j]) * 0.5);
-        } else {
-            f.MST[c] = (F)U0[pidx(g, i, 0, k)];
-            f.MST[c + 2 * g.FS] = (F)U0[pidx(g, i, 0, k)];
-        }
-        f.MST[c + g.FS] = (F)((U0[c] + U0[pidx(g, im, j, k)] + U0[pidx(g, i, j, km)] + U0[pidx(g, im, j, km)]) * 0.5 * 0.5);
-        if (j == M) {
-            const long long ct = pidx(g, i, M + 1, k);
-            f.DST[ct + g.FS] = (F)R[ct];
-            f.MST[ct] = (F)U0[ct];
-            f.MST[ct + 2 * g.FS] = (F)U0[ct];
-        }
+        F d1, d2, d3;
+        io_props_point(g, f, i, j, k, d1, d2, d3);
     }
 }
 
