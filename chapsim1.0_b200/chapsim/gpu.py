@@ -313,7 +313,10 @@ class ChannelTG:
         domain (0 explicit, 1 Crank-Nicolson); the TG domain accepts 0 only.
         pdl: launch the step's kernels with programmatic dependent launch."""
         self.lib = load_library()
-        self.choice = 0  # variant bits in use (chapsim_autotune); the library starts with all zero
+        # variant bits in use (chapsim_autotune): what the library starts with
+        self.choice = 0
+        if precision == "fp64" and self.IDOMAIN == 1:
+            self.choice = 64 | 256 | (8 if plane_in_one_block(setup.L, setup.N, precision) else 0)
         if precision not in PRECISIONS:
             raise ValueError(f"precision must be one of {sorted(PRECISIONS)}")
         self.precision = precision

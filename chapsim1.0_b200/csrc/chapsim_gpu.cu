@@ -531,6 +531,10 @@ int configure_kernels(chapsim_ctx* ctx) {
     ctx->zs_tw = ctx->prec != CHAPSIM_PREC_MIXED ? 16 : 32;
     int rc = ctx->prec == CHAPSIM_PREC_MIXED ? configure_momentum<float>(ctx) : configure_momentum<double>(ctx);
     if (rc) return rc;
+    // and the fused plane transforms in FP64 where a plane fits one block (chained / fused pressure stage:
+    // 21.6 / 19.6 us at 64^3, 84.2 / 71.0 at 128^3, 162 / 143 at 192 x 256 x 96); the cluster form is slower
+    // than the chained transforms (303 / 426 at 256 x 128 x 256)
+    if (ctx->domain == 1 && ctx->prec != CHAPSIM_PREC_MIXED && plane_fft_ok<double2>(g)) ctx->plane_kind = 1;
     // the FP64 spectral stage serves the standalone Poisson solve and the main domain in every precision
     DISPATCH_FFT(g.L, CK(set_smem(k_fftx_inv<FN1, FN2, double2>, smem_px(g))));
     DISPATCH_FFT(g.L, CK(set_smem(k_fftx_from_rhs<FN1, FN2>, smem_px(g))));
@@ -1204,6 +1208,16 @@ int chapsim_gpu_init(const chapsim_grid_t* grid, const chapsim_coefs_t* cf, cons
     g.yz = ctx->yz;
     k_ysolve_zero_factors<<<1, 32, 0, ctx->stream>>>(g, ctx->yz);
     INIT_CK(cudaGetLastError());
+    if (ctx->prec == CHAPSIM_PREC_FP64 && !xio) {
+        // FP64 contexts start with the y-solve by affine scans: faster than the hybrid at every size measured
+        // (warp hybrid / scans: 12.7 / 6.3 us at 64^3, 43.0 / 21.1 at 128^3, 79.4 / 32.0 at 192 x 256 x 96,
+        // 449 / 264 at 384 x 256 x 384).  Mixed-precision contexts start with the hybrid: their FP32 fields
+        // are reproduced to the bit.
+        INIT_CK(cudaMalloc(&ctx->YF3, (size_t)g.LH * M * N * sizeof(double)));
+        k_ysolve_scan_factors<<<(int)(((long long)g.LH * N + 127) / 128), 128, 0, ctx->stream>>>(g, ctx->YF3);
+        INIT_CK(cudaGetLastError());
+        ctx->ysolve_kind = 4;
+    }
     // fields
     INIT_CK(cudaMalloc(&ctx->Q, (size_t)(3 * g.FS) * sizeof(double)));
     INIT_CK(cudaMalloc(&ctx->PR, (size_t)g.FS * sizeof(double)));

@@ -535,7 +535,9 @@ int chapsim_dump_write(chapsim_ctx_t* ctx, const char* path_prefix, int32_t iter
  * the z sweep with pair-interleaved 32- and 16-line tiles, the y sweep with
  * line-contiguous and pair-interleaved tiles, and the pressure stage with
  * the z transforms' wave-ahead requests.
- * CONVH0 is restored after the trial launches. */
+ * CONVH0 is restored after the trial launches.  Without the call a mixed-
+ * precision context runs with all bits 0, an FP64 one with bits 6 and 8, and
+ * bit 3 where a plane fits one block. */
 int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choice, float* ms);
 
 /* An ensemble of independent periodic channels (any grids and precisions, one
