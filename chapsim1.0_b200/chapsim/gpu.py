@@ -713,7 +713,7 @@ class ChannelIO(ChannelTG):
 
     def kernel_slots(self):
         mom = (["k_io_rhs_cn", "k_io_cn_xsweep", "k_io_cn_zysweep"] if self.ivisscheme
-               else ["k_io_divu", "k_io_rhs", "k_io_massflux"])
+               else ["k_io_divu" if self.precision == "mixed" else None, "k_io_rhs", "k_io_massflux"])
         eng = (["k_eng_rhs", "k_mlp_infer" if self.use_mlp else "k_eng_props", "k_eng_bc", "k_eng_state", None,
                 None] if self.thermal else [])
         sub = eng + mom + ["k_io_div_fftx", "k_fftz_fwd", "k_ysolve", "k_fftz_inv", "k_fftx_inv", "k_io_correct"]
@@ -837,7 +837,7 @@ class ChannelXinout(ChannelIO):
 
     def kernel_slots(self):
         fft = self.L in (32, 64, 96, 128, 192, 256, 384)  # the cosine transforms through the FFT
-        sub = ["k_xio_inlet", "k_xio_outlet_a", "k_xio_outlet_b", "k_xio_outlet_c", "k_io_divu", "k_io_rhs",
+        sub = ["k_xio_inlet", "k_xio_outlet_a", "k_xio_outlet_b", "k_xio_outlet_c", "k_io_rhs",
                "k_io_massflux", "k_xio_div_cosqf" if fft else "k_xio_div_dctx", "k_fftz_fwd", "k_xio_ysolve",
                "k_fftz_inv", "k_xio_cosqb" if fft else "k_xio_dctx_inv", "k_io_correct"]
         return ["k_io_cfl", "k_dt", "k_dt_pair"] + sub * 3

@@ -547,6 +547,10 @@ int configure_kernels(chapsim_ctx* ctx) {
     CK(set_smem(k_ysolve_2w<double2>, smem_ysolve_seq()));
     DISPATCH_FFT(g.N, CK(set_smem(k_fftz<-1, FN1, FN2, double2>, smem_fz(g))));
     DISPATCH_FFT(g.N, CK(set_smem(k_fftz<+1, FN1, FN2, double2>, smem_fz(g))));
+    if (ctx->domain >= 2) {
+        CK(set_smem(k_io_rhs_tile<false>, IT_SMEM));
+        CK(set_smem(k_io_rhs_tile<true>, IT_SMEM));
+    }
     if (ctx->domain == 2 && ctx->ivis) {
         DISPATCH_S(g.L / 32, CK(set_smem(k_io_cn_xsweep<S * 32 / cn_w<double>(), double>, smem_cn_x<double>(g.L))));
         DISPATCH_S(g.L / 32, CK(set_smem(k_io_cn_xsweep<S * 32 / cn_w<float>(), float>, smem_cn_x<float>(g.L))));
@@ -882,6 +886,18 @@ void launch_io_step_start(chapsim_ctx* ctx) {
     ctx->launches += 2;
 }
 
+// explicit right-hand sides of the main domain: the tile form in FP64, the flat one with FP32 storage
+template <bool CN>
+void launch_io_rhs(chapsim_ctx* ctx, const IoFields& f, int ns) {
+    const Geo& g = ctx->g;
+    const int chunk = io_tile_chunk(g, ctx->nsm);
+    k_io_rhs_tile<CN><<<io_tile_blocks(g, chunk), IT_NT, IT_SMEM, ctx->stream>>>(g, f, ctx->part_rhs, ctx->st, ns, chunk);
+}
+template <bool CN>
+void launch_io_rhs(chapsim_ctx* ctx, const IoFieldsT<float>& f, int ns) {
+    k_io_rhs<CN, float><<<ctx->io_grid, IO_NT, 0, ctx->stream>>>(ctx->g, f, ctx->part_rhs, ctx->st, ns);
+}
+
 template <typename F>
 void launch_io_substep_t(chapsim_ctx* ctx, int ns) {
     const Geo& g = ctx->g;
@@ -889,15 +905,18 @@ void launch_io_substep_t(chapsim_ctx* ctx, int ns) {
     if (ctx->thermal) launch_thermal_substep_t<F>(ctx, ns);
     IoFieldsT<F> f = io_fields_t<F>(ctx);
     if (!ctx->ivis) {
-        k_io_divu<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f);
+        if constexpr (sizeof(F) == 4) {  // (the FP64 kernel forms DivU itself)
+            k_io_divu<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f);
+            ctx->launches += 1;
+        }
         prof_mark(ctx);
-        k_io_rhs<false, F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->part_rhs, ctx->st, ns);
+        launch_io_rhs<false>(ctx, f, ns);
         prof_mark(ctx);
         k_io_massflux<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->st, ns);
         prof_mark(ctx);
     } else {
         // VISCOUS_PAR_EXPLT_* + RHS_MOM_EXPLICIT_io, then MOMFA_io's sweeps for all components
-        k_io_rhs<true, F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->part_rhs, ctx->st, ns);
+        launch_io_rhs<true>(ctx, f, ns);
         prof_mark(ctx);
         constexpr int XS = 32 / cn_w<F>();  // segment length over DISPATCH_S's n / 32
         dim3 gx((unsigned)((g.M * (long long)g.N + cn_xlines<F>() - 1) / cn_xlines<F>()), 3);
@@ -907,7 +926,7 @@ void launch_io_substep_t(chapsim_ctx* ctx, int ns) {
         DISPATCH_S(g.N / 32, (k_io_cn_zsweep<S * XS, F><<<gz, CN_NT, 0, s>>>(g, f, ctx->st, ns)));
         DISPATCH_S(g.M / 32, (k_io_cn_ysweep<S * XS, F><<<gy, CN_NT, 0, s>>>(g, f, ctx->st, ns)));
         prof_mark(ctx);
-        ctx->launches += 1;
+        ctx->launches += 2;
     }
     // the Poisson stage is FP64 in both precisions
     dim3 grp((g.M + PX_TJ - 1) / PX_TJ, g.N);
@@ -928,7 +947,7 @@ void launch_io_substep_t(chapsim_ctx* ctx, int ns) {
     prof_mark(ctx);
     k_io_correct<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->DPH, ctx->st, ns, ctx->ivis ? ctx->RHSLL : nullptr);
     prof_mark(ctx);
-    ctx->launches += 9;
+    ctx->launches += 8;
 }
 void launch_io_substep(chapsim_ctx* ctx, int ns) {
     if (io_mixed(ctx)) launch_io_substep_t<float>(ctx, ns);
@@ -967,9 +986,7 @@ void launch_xio_substep(chapsim_ctx* ctx, int ns) {
     k_xio_outlet_c<<<gout, XIO_NT, 0, s>>>(g, f, ctx->xio_part + 2 * gout, ctx->thermal ? ctx->xio_mpart : nullptr,
                                            ctx->io_grid, ctx->xio_state, ctx->st);
     prof_mark(ctx);
-    k_io_divu<double><<<ctx->io_grid, IO_NT, 0, s>>>(g, f);
-    prof_mark(ctx);
-    k_io_rhs<false, double><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->part_rhs, ctx->st, ns);
+    launch_io_rhs<false>(ctx, f, ns);
     prof_mark(ctx);
     k_io_massflux<double><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->st, ns);
     prof_mark(ctx);
@@ -1001,7 +1018,7 @@ void launch_xio_substep(chapsim_ctx* ctx, int ns) {
     prof_mark(ctx);
     k_io_correct<double><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->DPH, ctx->st, ns, nullptr);
     prof_mark(ctx);
-    ctx->launches += 13;
+    ctx->launches += 12;
 }
 
 // CFL_tg and CFL_io of one TG + main-domain step, then CFLMM = max of the two and the dt rule

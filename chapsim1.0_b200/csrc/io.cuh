@@ -155,273 +155,269 @@ __global__ void __launch_bounds__(IO_NT) k_io_divu(Geo g, IoFieldsT<F> f) {
 //     src/MASSFLUX_CALC_IO.f90:332-416), and 0 before that (MEMALLOCT.f90:209).
 //     It is therefore not computed.  The v row j = 1 is left unwritten; the
 //     Crank-Nicolson sweeps treat it as zero.
-template <bool CN, typename F>
-__global__ void __launch_bounds__(IO_NT, 2) k_io_rhs(Geo g, IoFieldsT<F> f, double* __restrict__ partial, DevState* __restrict__ st,
-                                                  int ns) {
-    __shared__ double sred[32];
-    __shared__ int is_last;
-    const int N = g.N;
-    const long long tot = io_points(g);
-    const long long FS = g.FS;
-    const double dt = st->dt, tg = g.tgam[ns], tr = g.troh[ns], ta = g.talp[ns];
+// The convection and viscous terms of one point: ex the explicit part, im the implicit one (CN only).
+// A gives the fields at the point's neighbours: q, g, ms (component, di, dj, dk), u0, u, dv (di, dj, dk).
+struct IoRow { double wffj, wfbj, wffp, wfbp, dyfij, dyfim, dycij, dycip; };  // y coefficients of row j
+__device__ __forceinline__ IoRow io_row(const Geo& g, int j) {
+    return {g.wff[j], g.wfb[j], g.wff[j + 1], g.wfb[j + 1], g.dyfi[j], g.dyfi[j - 1], g.dyci[j], g.dyci[j + 1]};
+}
+template <bool CN, class A>
+__device__ __forceinline__ void io_rhs_terms(const Geo& g, const IoRow& y, const A& a, int j, double& ex1, double& ex2, double& ex3,
+                                             double& im1, double& im2, double& im3) {
     const double cv = g.cvisc;
-    const F* G = f.G;
-    const F* Q = f.Q;
-    const double* U0 = f.MU0;
-    const double* U = f.MU;
-    const F* MS = f.MST;
-    const F* DV = f.DIVU;
-    const F* PR = f.PR;
-    double bulk = 0.0;
-    for (long long t = (long long)blockIdx.x * IO_NT + threadIdx.x; t < tot; t += (long long)gridDim.x * IO_NT) {
-        int i, j, k;
-        io_decode(g, t, i, j, k);
-        const int ip = xpn(g, i), im = xmn(g, i), kp = wrapp(k, N), km = wrapm(k, N);
-        const int jp = j + 1, jm = j - 1;
-        const long long c = pidx(g, i, j, k);
-        const long long cip = pidx(g, ip, j, k), cim = pidx(g, im, j, k);
-        const long long cjp = pidx(g, i, jp, k), cjm = pidx(g, i, jm, k);
-        const long long ckp = pidx(g, i, j, kp), ckm = pidx(g, i, j, km);
-        const double wffj = g.wff[j], wfbj = g.wfb[j], wffp = g.wff[jp], wfbp = g.wfb[jp];
-        const double dyfij = g.dyfi[j], dycij = g.dyci[j], dycip = g.dyci[jp];
-        // -------- x momentum: CONVECTION_X_io + viscous terms --------
-        double ex1, ex2 = 0.0, ex3, im1 = 0.0, im2 = 0.0, im3 = 0.0;
-        {
-            const double H11F = (G[cip] + G[c]) * (Q[cip] + Q[c]);
-            const double H11B = (G[c] + G[cim]) * (Q[c] + Q[cim]);
-            const double H11 = (H11F - H11B) * (g.dxi * 0.5 * 0.5);
-            const double H12F = (G[cjp + FS] + G[pidx(g, im, jp, k) + FS]) * (wffp * Q[cjp] + wfbp * Q[c]);
-            const double H12B = (G[c + FS] + G[cim + FS]) * (wffj * Q[c] + wfbj * Q[cjm]);
-            const double H12 = (H12F - H12B) * (dyfij * 0.5 * 1.0);
-            const double H13F = (G[ckp + 2 * FS] + G[pidx(g, im, j, kp) + 2 * FS]) * (Q[ckp] + Q[c]);
-            const double H13B = (G[c + 2 * FS] + G[cim + 2 * FS]) * (Q[c] + Q[ckm]);
-            const double H13 = (H13F - H13B) * ((g.dzi * 0.5 * 0.5) * 1.0);
-            ex1 = -(H11 + H12 + H13);
-            if constexpr (!CN) {
-                double DUDX = (Q[cip] - Q[c]) * g.dxi;
-                const double T11F = 0.5 * (U0[c] + U0[c]) * (DUDX - DV[c]);
-                DUDX = (Q[c] - Q[cim]) * g.dxi;
-                const double T11B = 0.5 * (U0[cim] + U0[cim]) * (DUDX - DV[cim]);
-                const double D11 = (T11F - T11B) * (2.0 * g.dxi * cv);
-                double DUDY = (Q[cjp] - Q[c]) * dycip / 1.0;
-                double DVDX = (Q[cjp + FS] - Q[pidx(g, im, jp, k) + FS]) * g.dxi;
-                const double T12F = MS[cjp] * (DUDY + DVDX);
-                DUDY = (Q[c] - Q[cjm]) * dycij / 1.0;
-                DVDX = (Q[c + FS] - Q[cim + FS]) * g.dxi;
-                const double T12B = MS[c] * (DUDY + DVDX);
-                const double D12 = (T12F - T12B) * (dyfij * cv * 1.0);
-                double DUDZ = (Q[ckp] - Q[c]) * g.dzi;
-                double DWDX = (Q[ckp + 2 * FS] - Q[pidx(g, im, j, kp) + 2 * FS]) * g.dxi;
-                const double T13F = MS[ckp + FS] * (DUDZ + DWDX);
-                DUDZ = (Q[c] - Q[ckm]) * g.dzi;
-                DWDX = (Q[c + 2 * FS] - Q[cim + 2 * FS]) * g.dxi;
-                const double T13B = MS[c + FS] * (DUDZ + DWDX);
-                const double D13 = (T13F - T13B) * ((g.dzi * cv) * 1.0);
-                ex1 = ex1 + D11 + D12 + D13;
-            } else {
-                const double coe1 = -2.0 / 3.0 * g.dxi * cv;
-                double DUDX = (Q[cip] - Q[c]) * g.dxi;
-                double DVDY = (Q[cjp + FS] - Q[c + FS]) * dyfij * 1.0;
-                double DWDZ = (Q[ckp + 2 * FS] - Q[c + 2 * FS]) * g.dzi * 1.0;
-                const double F_EX11 = U[c] * (DVDY + DWDZ), F_IM11 = U[c] * DUDX;
-                DUDX = (Q[c] - Q[cim]) * g.dxi;
-                DVDY = (Q[pidx(g, im, jp, k) + FS] - Q[cim + FS]) * dyfij * 1.0;
-                DWDZ = (Q[pidx(g, im, j, kp) + 2 * FS] - Q[cim + 2 * FS]) * g.dzi * 1.0;
-                const double B_EX11 = U[cim] * (DVDY + DWDZ), B_IM11 = U[cim] * DUDX;
-                const double D11_EX = (F_EX11 - B_EX11) * coe1;
-                const double D11_IM = (F_IM11 - B_IM11) * coe1 * (-2.0);
-                const double coe2 = dyfij * cv * 1.0;
-                double DVDX = (Q[cjp + FS] - Q[pidx(g, im, jp, k) + FS]) * g.dxi;
-                double DUDY = (Q[cjp] - Q[c]) * dycip / 1.0;
-                const double F_EX12 = MS[cjp] * DVDX, F_IM12 = MS[cjp] * DUDY;
-                DUDY = (Q[c] - Q[cjm]) * dycij / 1.0;
-                DVDX = (Q[c + FS] - Q[cim + FS]) * g.dxi;
-                const double B_EX12 = MS[c] * DVDX, B_IM12 = MS[c] * DUDY;
-                const double D12_EX = (F_EX12 - B_EX12) * coe2;
-                const double D12_IM = (F_IM12 - B_IM12) * coe2;
-                const double coe32 = (g.dzi * cv) * 1.0;
-                double DUDZ = (Q[ckp] - Q[c]) * g.dzi;
-                double DWDX = (Q[ckp + 2 * FS] - Q[pidx(g, im, j, kp) + 2 * FS]) * g.dxi;
-                const double F_EX13 = MS[ckp + FS] * DWDX, F_IM13 = MS[ckp + FS] * DUDZ;
-                DUDZ = (Q[c] - Q[ckm]) * g.dzi;
-                DWDX = (Q[c + 2 * FS] - Q[cim + 2 * FS]) * g.dxi;
-                const double B_EX13 = MS[c + FS] * DWDX, B_IM13 = MS[c + FS] * DUDZ;
-                const double D13_EX = (F_EX13 - B_EX13) * coe32;
-                const double D13_IM = (F_IM13 - B_IM13) * coe32;
-                ex1 = D11_EX + D12_EX + D13_EX + ex1;
-                im1 = D11_IM + D12_IM + D13_IM;
-            }
+    const double wffj = y.wffj, wfbj = y.wfbj, wffp = y.wffp, wfbp = y.wfbp;
+    const double dyfij = y.dyfij, dyfim = y.dyfim, dycij = y.dycij, dycip = y.dycip;
+    ex2 = im1 = im2 = im3 = 0.0;
+    // -------- x momentum: CONVECTION_X_io + viscous terms --------
+    {
+        const double H11F = (a.g(0, 1, 0, 0) + a.g(0, 0, 0, 0)) * (a.q(0, 1, 0, 0) + a.q(0, 0, 0, 0));
+        const double H11B = (a.g(0, 0, 0, 0) + a.g(0, -1, 0, 0)) * (a.q(0, 0, 0, 0) + a.q(0, -1, 0, 0));
+        const double H11 = (H11F - H11B) * (g.dxi * 0.5 * 0.5);
+        const double H12F = (a.g(1, 0, 1, 0) + a.g(1, -1, 1, 0)) * (wffp * a.q(0, 0, 1, 0) + wfbp * a.q(0, 0, 0, 0));
+        const double H12B = (a.g(1, 0, 0, 0) + a.g(1, -1, 0, 0)) * (wffj * a.q(0, 0, 0, 0) + wfbj * a.q(0, 0, -1, 0));
+        const double H12 = (H12F - H12B) * (dyfij * 0.5 * 1.0);
+        const double H13F = (a.g(2, 0, 0, 1) + a.g(2, -1, 0, 1)) * (a.q(0, 0, 0, 1) + a.q(0, 0, 0, 0));
+        const double H13B = (a.g(2, 0, 0, 0) + a.g(2, -1, 0, 0)) * (a.q(0, 0, 0, 0) + a.q(0, 0, 0, -1));
+        const double H13 = (H13F - H13B) * ((g.dzi * 0.5 * 0.5) * 1.0);
+        ex1 = -(H11 + H12 + H13);
+        if constexpr (!CN) {
+            double DUDX = (a.q(0, 1, 0, 0) - a.q(0, 0, 0, 0)) * g.dxi;
+            const double T11F = 0.5 * (a.u0(0, 0, 0) + a.u0(0, 0, 0)) * (DUDX - a.dv(0, 0, 0));
+            DUDX = (a.q(0, 0, 0, 0) - a.q(0, -1, 0, 0)) * g.dxi;
+            const double T11B = 0.5 * (a.u0(-1, 0, 0) + a.u0(-1, 0, 0)) * (DUDX - a.dv(-1, 0, 0));
+            const double D11 = (T11F - T11B) * (2.0 * g.dxi * cv);
+            double DUDY = (a.q(0, 0, 1, 0) - a.q(0, 0, 0, 0)) * dycip / 1.0;
+            double DVDX = (a.q(1, 0, 1, 0) - a.q(1, -1, 1, 0)) * g.dxi;
+            const double T12F = a.ms(0, 0, 1, 0) * (DUDY + DVDX);
+            DUDY = (a.q(0, 0, 0, 0) - a.q(0, 0, -1, 0)) * dycij / 1.0;
+            DVDX = (a.q(1, 0, 0, 0) - a.q(1, -1, 0, 0)) * g.dxi;
+            const double T12B = a.ms(0, 0, 0, 0) * (DUDY + DVDX);
+            const double D12 = (T12F - T12B) * (dyfij * cv * 1.0);
+            double DUDZ = (a.q(0, 0, 0, 1) - a.q(0, 0, 0, 0)) * g.dzi;
+            double DWDX = (a.q(2, 0, 0, 1) - a.q(2, -1, 0, 1)) * g.dxi;
+            const double T13F = a.ms(1, 0, 0, 1) * (DUDZ + DWDX);
+            DUDZ = (a.q(0, 0, 0, 0) - a.q(0, 0, 0, -1)) * g.dzi;
+            DWDX = (a.q(2, 0, 0, 0) - a.q(2, -1, 0, 0)) * g.dxi;
+            const double T13B = a.ms(1, 0, 0, 0) * (DUDZ + DWDX);
+            const double D13 = (T13F - T13B) * ((g.dzi * cv) * 1.0);
+            ex1 = ex1 + D11 + D12 + D13;
+        } else {
+            const double coe1 = -2.0 / 3.0 * g.dxi * cv;
+            double DUDX = (a.q(0, 1, 0, 0) - a.q(0, 0, 0, 0)) * g.dxi;
+            double DVDY = (a.q(1, 0, 1, 0) - a.q(1, 0, 0, 0)) * dyfij * 1.0;
+            double DWDZ = (a.q(2, 0, 0, 1) - a.q(2, 0, 0, 0)) * g.dzi * 1.0;
+            const double F_EX11 = a.u(0, 0, 0) * (DVDY + DWDZ), F_IM11 = a.u(0, 0, 0) * DUDX;
+            DUDX = (a.q(0, 0, 0, 0) - a.q(0, -1, 0, 0)) * g.dxi;
+            DVDY = (a.q(1, -1, 1, 0) - a.q(1, -1, 0, 0)) * dyfij * 1.0;
+            DWDZ = (a.q(2, -1, 0, 1) - a.q(2, -1, 0, 0)) * g.dzi * 1.0;
+            const double B_EX11 = a.u(-1, 0, 0) * (DVDY + DWDZ), B_IM11 = a.u(-1, 0, 0) * DUDX;
+            const double D11_EX = (F_EX11 - B_EX11) * coe1;
+            const double D11_IM = (F_IM11 - B_IM11) * coe1 * (-2.0);
+            const double coe2 = dyfij * cv * 1.0;
+            double DVDX = (a.q(1, 0, 1, 0) - a.q(1, -1, 1, 0)) * g.dxi;
+            double DUDY = (a.q(0, 0, 1, 0) - a.q(0, 0, 0, 0)) * dycip / 1.0;
+            const double F_EX12 = a.ms(0, 0, 1, 0) * DVDX, F_IM12 = a.ms(0, 0, 1, 0) * DUDY;
+            DUDY = (a.q(0, 0, 0, 0) - a.q(0, 0, -1, 0)) * dycij / 1.0;
+            DVDX = (a.q(1, 0, 0, 0) - a.q(1, -1, 0, 0)) * g.dxi;
+            const double B_EX12 = a.ms(0, 0, 0, 0) * DVDX, B_IM12 = a.ms(0, 0, 0, 0) * DUDY;
+            const double D12_EX = (F_EX12 - B_EX12) * coe2;
+            const double D12_IM = (F_IM12 - B_IM12) * coe2;
+            const double coe32 = (g.dzi * cv) * 1.0;
+            double DUDZ = (a.q(0, 0, 0, 1) - a.q(0, 0, 0, 0)) * g.dzi;
+            double DWDX = (a.q(2, 0, 0, 1) - a.q(2, -1, 0, 1)) * g.dxi;
+            const double F_EX13 = a.ms(1, 0, 0, 1) * DWDX, F_IM13 = a.ms(1, 0, 0, 1) * DUDZ;
+            DUDZ = (a.q(0, 0, 0, 0) - a.q(0, 0, 0, -1)) * g.dzi;
+            DWDX = (a.q(2, 0, 0, 0) - a.q(2, -1, 0, 0)) * g.dxi;
+            const double B_EX13 = a.ms(1, 0, 0, 0) * DWDX, B_IM13 = a.ms(1, 0, 0, 0) * DUDZ;
+            const double D13_EX = (F_EX13 - B_EX13) * coe32;
+            const double D13_IM = (F_IM13 - B_IM13) * coe32;
+            ex1 = D11_EX + D12_EX + D13_EX + ex1;
+            im1 = D11_IM + D12_IM + D13_IM;
         }
-        // -------- y momentum (j >= 2) --------
-        if (j >= 2) {
-            const double H21F = (wffj * G[cip] + wfbj * G[pidx(g, ip, jm, k)]) * (Q[cip + FS] + Q[c + FS]);
-            const double H21B = (wffj * G[c] + wfbj * G[cjm]) * (Q[c + FS] + Q[cim + FS]);
-            const double H21 = (H21F - H21B) * (g.dxi * 0.5);
-            const double H22F = (G[cjp + FS] + G[c + FS]) * (Q[cjp + FS] * 1.0 + Q[c + FS] * 1.0);
-            const double H22B = (G[c + FS] + G[cjm + FS]) * (Q[c + FS] * 1.0 + Q[cjm + FS] * 1.0);
-            const double H22 = (H22F - H22B) * (dycij * 0.5 * 0.5);
-            const double H23F = (wffj * G[ckp + 2 * FS] * 1.0 + wfbj * G[pidx(g, i, jm, kp) + 2 * FS] * 1.0) * (Q[ckp + FS] + Q[c + FS]);
-            const double H23B = (wffj * G[c + 2 * FS] * 1.0 + wfbj * G[cjm + 2 * FS] * 1.0) * (Q[c + FS] + Q[ckm + FS]);
-            const double H23 = (H23F - H23B) * ((g.dzi * 0.5) * 1.0);
-            ex2 = -(H21 + H22 + H23);
-            if constexpr (!CN) {
-                double DVDY = (Q[cjp + FS] - Q[c + FS]) * dyfij;
-                const double T22F = 0.5 * (U0[c] + U0[c]) * (DVDY - DV[c]);
-                DVDY = (Q[c + FS] - Q[cjm + FS]) * g.dyfi[jm];
-                const double T22B = 0.5 * (U0[cjm] + U0[cjm]) * (DVDY - DV[cjm]);
-                const double D22 = (T22F - T22B) * (2.0 * dycij * cv);
-                double DVDX = (Q[cip + FS] - Q[c + FS]) * g.dxi;
-                double DUDY = (Q[cip] - Q[pidx(g, ip, jm, k)]) * dycij;
-                const double T21F = MS[cip] * (DVDX + DUDY);
-                DVDX = (Q[c + FS] - Q[cim + FS]) * g.dxi;
-                DUDY = (Q[c] - Q[cjm]) * dycij;
-                const double T21B = MS[c] * (DVDX + DUDY);
-                const double D21 = (T21F - T21B) * (g.dxi * cv);
-                double DVDZ = (Q[ckp + FS] - Q[c + FS]) * g.dzi;
-                double DWDY = (Q[ckp + 2 * FS] - Q[pidx(g, i, jm, kp) + 2 * FS]) * dycij;
-                const double T23F = MS[ckp + 2 * FS] * (DVDZ + DWDY);
-                DVDZ = (Q[c + FS] - Q[ckm + FS]) * g.dzi;
-                DWDY = (Q[c + 2 * FS] - Q[cjm + 2 * FS]) * dycij;
-                const double T23B = MS[c + 2 * FS] * (DVDZ + DWDY);
-                const double D23 = (T23F - T23B) * (g.dzi * cv);
-                ex2 = ex2 + D21 + D22 + D23;
-            } else {
-                const double coe2 = -2.0 / 3.0 * dycij * cv;
-                double DUDX = (Q[cip] - Q[c]) * g.dxi;
-                double DVDY = (Q[cjp + FS] - Q[c + FS]) * dyfij;
-                double DWDZ = (Q[ckp + 2 * FS] - Q[c + 2 * FS]) * g.dzi;
-                const double F_EX22 = U[c] * (DUDX + DWDZ), F_IM22 = U[c] * DVDY;
-                DUDX = (Q[pidx(g, ip, jm, k)] - Q[cjm]) * g.dxi;
-                DVDY = (Q[c + FS] - Q[cjm + FS]) * g.dyfi[jm];
-                DWDZ = (Q[pidx(g, i, jm, kp) + 2 * FS] - Q[cjm + 2 * FS]) * g.dzi;
-                const double B_EX22 = U[cjm] * (DUDX + DWDZ), B_IM22 = U[cjm] * DVDY;
-                const double D22_EX = (F_EX22 - B_EX22) * coe2;
-                const double D22_IM = (F_IM22 - B_IM22) * coe2 * (-2.0);
-                const double coe1 = g.dxi * cv;
-                double DVDX = (Q[cip + FS] - Q[c + FS]) * g.dxi;
-                double DUDY = (Q[cip] - Q[pidx(g, ip, jm, k)]) * dycij;
-                const double F_EX21 = MS[cip] * DUDY, F_IM21 = MS[cip] * DVDX;
-                DVDX = (Q[c + FS] - Q[cim + FS]) * g.dxi;
-                DUDY = (Q[c] - Q[cjm]) * dycij;
-                const double B_EX21 = MS[c] * DUDY, B_IM21 = MS[c] * DVDX;
-                const double D21_EX = (F_EX21 - B_EX21) * coe1;
-                const double D21_IM = (F_IM21 - B_IM21) * coe1;
-                const double coe3 = g.dzi * cv;
-                double DVDZ = (Q[ckp + FS] - Q[c + FS]) * g.dzi;
-                double DWDY = (Q[ckp + 2 * FS] - Q[pidx(g, i, jm, kp) + 2 * FS]) * dycij;
-                const double F_EX23 = MS[ckp + 2 * FS] * DWDY, F_IM23 = MS[ckp + 2 * FS] * DVDZ;
-                DVDZ = (Q[c + FS] - Q[ckm + FS]) * g.dzi;
-                DWDY = (Q[c + 2 * FS] - Q[cjm + 2 * FS]) * dycij;
-                const double B_EX23 = MS[c + 2 * FS] * DWDY, B_IM23 = MS[c + 2 * FS] * DVDZ;
-                const double D23_EX = (F_EX23 - B_EX23) * coe3;
-                const double D23_IM = (F_IM23 - B_IM23) * coe3;
-                ex2 = D21_EX + D22_EX + D23_EX + ex2;
-                im2 = D21_IM + D22_IM + D23_IM;
-            }
-        }
-        // -------- z momentum --------
-        {
-            const double H31F = (G[cip] + G[pidx(g, ip, j, km)]) * (Q[cip + 2 * FS] + Q[c + 2 * FS]);
-            const double H31B = (G[c] + G[ckm]) * (Q[c + 2 * FS] + Q[cim + 2 * FS]);
-            const double H31 = (H31F - H31B) * (g.dxi * 0.5 * 0.5);
-            const double H32F = (G[cjp + FS] + G[pidx(g, i, jp, km) + FS]) * (wffp * Q[cjp + 2 * FS] * 1.0 + wfbp * Q[c + 2 * FS] * 1.0);
-            const double H32B = (G[c + FS] + G[ckm + FS]) * (wffj * Q[c + 2 * FS] * 1.0 + wfbj * Q[cjm + 2 * FS] * 1.0);
-            const double H32 = (H32F - H32B) * (dyfij * 0.5);
-            const double H33F = (G[ckp + 2 * FS] + G[c + 2 * FS]) * (Q[ckp + 2 * FS] + Q[c + 2 * FS]);
-            const double H33B = (G[c + 2 * FS] + G[ckm + 2 * FS]) * (Q[c + 2 * FS] + Q[ckm + 2 * FS]);
-            const double H33 = (H33F - H33B) * ((g.dzi * 0.5 * 0.5) * 1.0);
-            ex3 = -(H31 + H32 + H33);
-            if constexpr (!CN) {
-                double DWDZ = (Q[ckp + 2 * FS] - Q[c + 2 * FS]) * g.dzi;
-                const double T33F = 0.5 * (U0[c] + U0[c]) * (DWDZ - DV[c]);
-                DWDZ = (Q[c + 2 * FS] - Q[ckm + 2 * FS]) * g.dzi;
-                const double T33B = 0.5 * (U0[ckm] + U0[ckm]) * (DWDZ - DV[ckm]);
-                const double D33 = (T33F - T33B) * (2.0 * g.dzi * cv);
-                double DWDX = (Q[cip + 2 * FS] - Q[c + 2 * FS]) * g.dxi;
-                double DUDZ = (Q[cip] - Q[pidx(g, ip, j, km)]) * g.dzi;
-                const double T31F = MS[cip + FS] * (DWDX + DUDZ);
-                DWDX = (Q[c + 2 * FS] - Q[cim + 2 * FS]) * g.dxi;
-                DUDZ = (Q[c] - Q[ckm]) * g.dzi;
-                const double T31B = MS[c + FS] * (DWDX + DUDZ);
-                const double D31 = (T31F - T31B) * (g.dxi * cv);
-                double DWDY = (Q[cjp + 2 * FS] - Q[c + 2 * FS]) * dycip;
-                double DVDZ = (Q[cjp + FS] - Q[pidx(g, i, jp, km) + FS]) * g.dzi;
-                const double T32F = MS[cjp + 2 * FS] * (DWDY + DVDZ);
-                DWDY = (Q[c + 2 * FS] - Q[cjm + 2 * FS]) * dycij;
-                DVDZ = (Q[c + FS] - Q[ckm + FS]) * g.dzi;
-                const double T32B = MS[c + 2 * FS] * (DWDY + DVDZ);
-                const double D32 = (T32F - T32B) * (dyfij * cv);
-                ex3 = ex3 + D31 + D32 + D33;
-            } else {
-                const double coe3 = -2.0 / 3.0 * g.dzi * cv;
-                double DUDX = (Q[cip] - Q[c]) * g.dxi;
-                double DVDY = (Q[cjp + FS] - Q[c + FS]) * dyfij;
-                double DWDZ = (Q[ckp + 2 * FS] - Q[c + 2 * FS]) * g.dzi;
-                const double F_EX33 = U[c] * (DUDX + DVDY), F_IM33 = U[c] * DWDZ;
-                DUDX = (Q[pidx(g, ip, j, km)] - Q[ckm]) * g.dxi;
-                DVDY = (Q[pidx(g, i, jp, km) + FS] - Q[ckm + FS]) * dyfij;
-                DWDZ = (Q[c + 2 * FS] - Q[ckm + 2 * FS]) * g.dzi;
-                const double B_EX33 = U[ckm] * (DUDX + DVDY), B_IM33 = U[ckm] * DWDZ;
-                const double D33_EX = (F_EX33 - B_EX33) * coe3;
-                const double D33_IM = (F_IM33 - B_IM33) * coe3 * (-2.0);
-                const double coe1 = g.dxi * cv;
-                double DWDX = (Q[cip + 2 * FS] - Q[c + 2 * FS]) * g.dxi;
-                double DUDZ = (Q[cip] - Q[pidx(g, ip, j, km)]) * g.dzi;
-                const double F_EX31 = MS[cip + FS] * DUDZ, F_IM31 = MS[cip + FS] * DWDX;
-                DWDX = (Q[c + 2 * FS] - Q[cim + 2 * FS]) * g.dxi;
-                DUDZ = (Q[c] - Q[ckm]) * g.dzi;
-                const double B_EX31 = MS[c + FS] * DUDZ, B_IM31 = MS[c + FS] * DWDX;
-                const double D31_EX = (F_EX31 - B_EX31) * coe1;
-                const double D31_IM = (F_IM31 - B_IM31) * coe1;
-                const double coe2 = dyfij * cv;
-                double DWDY = (Q[cjp + 2 * FS] - Q[c + 2 * FS]) * dycip;
-                double DVDZ = (Q[cjp + FS] - Q[pidx(g, i, jp, km) + FS]) * g.dzi;
-                const double F_EX32 = MS[cjp + 2 * FS] * DVDZ, F_IM32 = MS[cjp + 2 * FS] * DWDY;
-                DWDY = (Q[c + 2 * FS] - Q[cjm + 2 * FS]) * dycij;
-                DVDZ = (Q[c + FS] - Q[ckm + FS]) * g.dzi;
-                const double B_EX32 = MS[c + 2 * FS] * DVDZ, B_IM32 = MS[c + 2 * FS] * DWDY;
-                const double D32_EX = (F_EX32 - B_EX32) * coe2;
-                const double D32_IM = (F_IM32 - B_IM32) * coe2;
-                ex3 = D31_EX + D32_EX + D33_EX + ex3;
-                im3 = D31_IM + D32_IM + D33_IM;
-            }
-        }
-        // -------- RHS_MOM_EXPLICIT_io --------
-        const long long ii = io_iidx(g, i, j, k);
-        // with inflow the inlet face u(1) is a boundary value: its x-momentum RHS, EXPLT0 and
-        // G are left alone (NXI = 2, src/RHS_MOM_EXPLICIT_io.f90:35)
-        const bool ux = !(g.xo && i == 1);
-        const double e01 = f.EX0[ii], e02 = f.EX0[ii + g.FI], e03 = f.EX0[ii + 2 * g.FI];
-        const double pc = PR[c], pim = PR[cim], pjm = PR[cjm], pkm = PR[ckm];
-        const double coa = ta * dt;
-        // buoyancy (:161-226): D_STG * TALP*DT*F_A on the component |iGravity| (1/RNDI1 = 1/RCCI1 = 1)
-        const int ig = f.igrav < 0 ? -f.igrav : f.igrav;
-        const double cob = ta * dt * f.fa;
-        double r1 = (tg * ex1 + tr * e01) * dt;
-        if constexpr (CN) r1 = r1 + coa * im1;
-        r1 = r1 - io_pgm(f, c, cim, pc, pim, ta * dt * g.dxi);
-        if (ig == 1) r1 = r1 + f.DST[c] * cob;
-        double r3 = (tg * ex3 + tr * e03) * dt;
-        if constexpr (CN) r3 = r3 + coa * im3;
-        r3 = r3 - io_pgm(f, c, ckm, pc, pkm, ta * dt * g.dzi);
-        if (ig == 3) r3 = r3 + f.DST[c + 2 * FS] * (cob / 1.0);
-        if (ux) {
-            f.EX0[ii] = (F)ex1;
-            f.RHS[ii] = (F)r1;
-        }
-        f.EX0[ii + 2 * g.FI] = (F)ex3;
-        f.RHS[ii + 2 * g.FI] = (F)r3;
-        if (j >= 2) {
-            double r2 = (tg * ex2 + tr * e02) * dt;
-            if constexpr (CN) r2 = r2 + coa * im2;
-            r2 = r2 - io_pgm(f, c, cjm, pc, pjm, ta * dt * dycij / 1.0);
-            if (ig == 2) r2 = r2 + f.DST[c + FS] * (cob / 1.0);
-            f.EX0[ii + g.FI] = (F)ex2;
-            f.RHS[ii + g.FI] = (F)r2;
-        }
-        if (ux) bulk += r1 / dyfij / 1.0;
     }
-    double s = block_sum<IO_NT>(bulk, sred);
+    // -------- y momentum (j >= 2) --------
+    if (j >= 2) {
+        const double H21F = (wffj * a.g(0, 1, 0, 0) + wfbj * a.g(0, 1, -1, 0)) * (a.q(1, 1, 0, 0) + a.q(1, 0, 0, 0));
+        const double H21B = (wffj * a.g(0, 0, 0, 0) + wfbj * a.g(0, 0, -1, 0)) * (a.q(1, 0, 0, 0) + a.q(1, -1, 0, 0));
+        const double H21 = (H21F - H21B) * (g.dxi * 0.5);
+        const double H22F = (a.g(1, 0, 1, 0) + a.g(1, 0, 0, 0)) * (a.q(1, 0, 1, 0) * 1.0 + a.q(1, 0, 0, 0) * 1.0);
+        const double H22B = (a.g(1, 0, 0, 0) + a.g(1, 0, -1, 0)) * (a.q(1, 0, 0, 0) * 1.0 + a.q(1, 0, -1, 0) * 1.0);
+        const double H22 = (H22F - H22B) * (dycij * 0.5 * 0.5);
+        const double H23F = (wffj * a.g(2, 0, 0, 1) * 1.0 + wfbj * a.g(2, 0, -1, 1) * 1.0) * (a.q(1, 0, 0, 1) + a.q(1, 0, 0, 0));
+        const double H23B = (wffj * a.g(2, 0, 0, 0) * 1.0 + wfbj * a.g(2, 0, -1, 0) * 1.0) * (a.q(1, 0, 0, 0) + a.q(1, 0, 0, -1));
+        const double H23 = (H23F - H23B) * ((g.dzi * 0.5) * 1.0);
+        ex2 = -(H21 + H22 + H23);
+        if constexpr (!CN) {
+            double DVDY = (a.q(1, 0, 1, 0) - a.q(1, 0, 0, 0)) * dyfij;
+            const double T22F = 0.5 * (a.u0(0, 0, 0) + a.u0(0, 0, 0)) * (DVDY - a.dv(0, 0, 0));
+            DVDY = (a.q(1, 0, 0, 0) - a.q(1, 0, -1, 0)) * dyfim;
+            const double T22B = 0.5 * (a.u0(0, -1, 0) + a.u0(0, -1, 0)) * (DVDY - a.dv(0, -1, 0));
+            const double D22 = (T22F - T22B) * (2.0 * dycij * cv);
+            double DVDX = (a.q(1, 1, 0, 0) - a.q(1, 0, 0, 0)) * g.dxi;
+            double DUDY = (a.q(0, 1, 0, 0) - a.q(0, 1, -1, 0)) * dycij;
+            const double T21F = a.ms(0, 1, 0, 0) * (DVDX + DUDY);
+            DVDX = (a.q(1, 0, 0, 0) - a.q(1, -1, 0, 0)) * g.dxi;
+            DUDY = (a.q(0, 0, 0, 0) - a.q(0, 0, -1, 0)) * dycij;
+            const double T21B = a.ms(0, 0, 0, 0) * (DVDX + DUDY);
+            const double D21 = (T21F - T21B) * (g.dxi * cv);
+            double DVDZ = (a.q(1, 0, 0, 1) - a.q(1, 0, 0, 0)) * g.dzi;
+            double DWDY = (a.q(2, 0, 0, 1) - a.q(2, 0, -1, 1)) * dycij;
+            const double T23F = a.ms(2, 0, 0, 1) * (DVDZ + DWDY);
+            DVDZ = (a.q(1, 0, 0, 0) - a.q(1, 0, 0, -1)) * g.dzi;
+            DWDY = (a.q(2, 0, 0, 0) - a.q(2, 0, -1, 0)) * dycij;
+            const double T23B = a.ms(2, 0, 0, 0) * (DVDZ + DWDY);
+            const double D23 = (T23F - T23B) * (g.dzi * cv);
+            ex2 = ex2 + D21 + D22 + D23;
+        } else {
+            const double coe2 = -2.0 / 3.0 * dycij * cv;
+            double DUDX = (a.q(0, 1, 0, 0) - a.q(0, 0, 0, 0)) * g.dxi;
+            double DVDY = (a.q(1, 0, 1, 0) - a.q(1, 0, 0, 0)) * dyfij;
+            double DWDZ = (a.q(2, 0, 0, 1) - a.q(2, 0, 0, 0)) * g.dzi;
+            const double F_EX22 = a.u(0, 0, 0) * (DUDX + DWDZ), F_IM22 = a.u(0, 0, 0) * DVDY;
+            DUDX = (a.q(0, 1, -1, 0) - a.q(0, 0, -1, 0)) * g.dxi;
+            DVDY = (a.q(1, 0, 0, 0) - a.q(1, 0, -1, 0)) * dyfim;
+            DWDZ = (a.q(2, 0, -1, 1) - a.q(2, 0, -1, 0)) * g.dzi;
+            const double B_EX22 = a.u(0, -1, 0) * (DUDX + DWDZ), B_IM22 = a.u(0, -1, 0) * DVDY;
+            const double D22_EX = (F_EX22 - B_EX22) * coe2;
+            const double D22_IM = (F_IM22 - B_IM22) * coe2 * (-2.0);
+            const double coe1 = g.dxi * cv;
+            double DVDX = (a.q(1, 1, 0, 0) - a.q(1, 0, 0, 0)) * g.dxi;
+            double DUDY = (a.q(0, 1, 0, 0) - a.q(0, 1, -1, 0)) * dycij;
+            const double F_EX21 = a.ms(0, 1, 0, 0) * DUDY, F_IM21 = a.ms(0, 1, 0, 0) * DVDX;
+            DVDX = (a.q(1, 0, 0, 0) - a.q(1, -1, 0, 0)) * g.dxi;
+            DUDY = (a.q(0, 0, 0, 0) - a.q(0, 0, -1, 0)) * dycij;
+            const double B_EX21 = a.ms(0, 0, 0, 0) * DUDY, B_IM21 = a.ms(0, 0, 0, 0) * DVDX;
+            const double D21_EX = (F_EX21 - B_EX21) * coe1;
+            const double D21_IM = (F_IM21 - B_IM21) * coe1;
+            const double coe3 = g.dzi * cv;
+            double DVDZ = (a.q(1, 0, 0, 1) - a.q(1, 0, 0, 0)) * g.dzi;
+            double DWDY = (a.q(2, 0, 0, 1) - a.q(2, 0, -1, 1)) * dycij;
+            const double F_EX23 = a.ms(2, 0, 0, 1) * DWDY, F_IM23 = a.ms(2, 0, 0, 1) * DVDZ;
+            DVDZ = (a.q(1, 0, 0, 0) - a.q(1, 0, 0, -1)) * g.dzi;
+            DWDY = (a.q(2, 0, 0, 0) - a.q(2, 0, -1, 0)) * dycij;
+            const double B_EX23 = a.ms(2, 0, 0, 0) * DWDY, B_IM23 = a.ms(2, 0, 0, 0) * DVDZ;
+            const double D23_EX = (F_EX23 - B_EX23) * coe3;
+            const double D23_IM = (F_IM23 - B_IM23) * coe3;
+            ex2 = D21_EX + D22_EX + D23_EX + ex2;
+            im2 = D21_IM + D22_IM + D23_IM;
+        }
+    }
+    // -------- z momentum --------
+    {
+        const double H31F = (a.g(0, 1, 0, 0) + a.g(0, 1, 0, -1)) * (a.q(2, 1, 0, 0) + a.q(2, 0, 0, 0));
+        const double H31B = (a.g(0, 0, 0, 0) + a.g(0, 0, 0, -1)) * (a.q(2, 0, 0, 0) + a.q(2, -1, 0, 0));
+        const double H31 = (H31F - H31B) * (g.dxi * 0.5 * 0.5);
+        const double H32F = (a.g(1, 0, 1, 0) + a.g(1, 0, 1, -1)) * (wffp * a.q(2, 0, 1, 0) * 1.0 + wfbp * a.q(2, 0, 0, 0) * 1.0);
+        const double H32B = (a.g(1, 0, 0, 0) + a.g(1, 0, 0, -1)) * (wffj * a.q(2, 0, 0, 0) * 1.0 + wfbj * a.q(2, 0, -1, 0) * 1.0);
+        const double H32 = (H32F - H32B) * (dyfij * 0.5);
+        const double H33F = (a.g(2, 0, 0, 1) + a.g(2, 0, 0, 0)) * (a.q(2, 0, 0, 1) + a.q(2, 0, 0, 0));
+        const double H33B = (a.g(2, 0, 0, 0) + a.g(2, 0, 0, -1)) * (a.q(2, 0, 0, 0) + a.q(2, 0, 0, -1));
+        const double H33 = (H33F - H33B) * ((g.dzi * 0.5 * 0.5) * 1.0);
+        ex3 = -(H31 + H32 + H33);
+        if constexpr (!CN) {
+            double DWDZ = (a.q(2, 0, 0, 1) - a.q(2, 0, 0, 0)) * g.dzi;
+            const double T33F = 0.5 * (a.u0(0, 0, 0) + a.u0(0, 0, 0)) * (DWDZ - a.dv(0, 0, 0));
+            DWDZ = (a.q(2, 0, 0, 0) - a.q(2, 0, 0, -1)) * g.dzi;
+            const double T33B = 0.5 * (a.u0(0, 0, -1) + a.u0(0, 0, -1)) * (DWDZ - a.dv(0, 0, -1));
+            const double D33 = (T33F - T33B) * (2.0 * g.dzi * cv);
+            double DWDX = (a.q(2, 1, 0, 0) - a.q(2, 0, 0, 0)) * g.dxi;
+            double DUDZ = (a.q(0, 1, 0, 0) - a.q(0, 1, 0, -1)) * g.dzi;
+            const double T31F = a.ms(1, 1, 0, 0) * (DWDX + DUDZ);
+            DWDX = (a.q(2, 0, 0, 0) - a.q(2, -1, 0, 0)) * g.dxi;
+            DUDZ = (a.q(0, 0, 0, 0) - a.q(0, 0, 0, -1)) * g.dzi;
+            const double T31B = a.ms(1, 0, 0, 0) * (DWDX + DUDZ);
+            const double D31 = (T31F - T31B) * (g.dxi * cv);
+            double DWDY = (a.q(2, 0, 1, 0) - a.q(2, 0, 0, 0)) * dycip;
+            double DVDZ = (a.q(1, 0, 1, 0) - a.q(1, 0, 1, -1)) * g.dzi;
+            const double T32F = a.ms(2, 0, 1, 0) * (DWDY + DVDZ);
+            DWDY = (a.q(2, 0, 0, 0) - a.q(2, 0, -1, 0)) * dycij;
+            DVDZ = (a.q(1, 0, 0, 0) - a.q(1, 0, 0, -1)) * g.dzi;
+            const double T32B = a.ms(2, 0, 0, 0) * (DWDY + DVDZ);
+            const double D32 = (T32F - T32B) * (dyfij * cv);
+            ex3 = ex3 + D31 + D32 + D33;
+        } else {
+            const double coe3 = -2.0 / 3.0 * g.dzi * cv;
+            double DUDX = (a.q(0, 1, 0, 0) - a.q(0, 0, 0, 0)) * g.dxi;
+            double DVDY = (a.q(1, 0, 1, 0) - a.q(1, 0, 0, 0)) * dyfij;
+            double DWDZ = (a.q(2, 0, 0, 1) - a.q(2, 0, 0, 0)) * g.dzi;
+            const double F_EX33 = a.u(0, 0, 0) * (DUDX + DVDY), F_IM33 = a.u(0, 0, 0) * DWDZ;
+            DUDX = (a.q(0, 1, 0, -1) - a.q(0, 0, 0, -1)) * g.dxi;
+            DVDY = (a.q(1, 0, 1, -1) - a.q(1, 0, 0, -1)) * dyfij;
+            DWDZ = (a.q(2, 0, 0, 0) - a.q(2, 0, 0, -1)) * g.dzi;
+            const double B_EX33 = a.u(0, 0, -1) * (DUDX + DVDY), B_IM33 = a.u(0, 0, -1) * DWDZ;
+            const double D33_EX = (F_EX33 - B_EX33) * coe3;
+            const double D33_IM = (F_IM33 - B_IM33) * coe3 * (-2.0);
+            const double coe1 = g.dxi * cv;
+            double DWDX = (a.q(2, 1, 0, 0) - a.q(2, 0, 0, 0)) * g.dxi;
+            double DUDZ = (a.q(0, 1, 0, 0) - a.q(0, 1, 0, -1)) * g.dzi;
+            const double F_EX31 = a.ms(1, 1, 0, 0) * DUDZ, F_IM31 = a.ms(1, 1, 0, 0) * DWDX;
+            DWDX = (a.q(2, 0, 0, 0) - a.q(2, -1, 0, 0)) * g.dxi;
+            DUDZ = (a.q(0, 0, 0, 0) - a.q(0, 0, 0, -1)) * g.dzi;
+            const double B_EX31 = a.ms(1, 0, 0, 0) * DUDZ, B_IM31 = a.ms(1, 0, 0, 0) * DWDX;
+            const double D31_EX = (F_EX31 - B_EX31) * coe1;
+            const double D31_IM = (F_IM31 - B_IM31) * coe1;
+            const double coe2 = dyfij * cv;
+            double DWDY = (a.q(2, 0, 1, 0) - a.q(2, 0, 0, 0)) * dycip;
+            double DVDZ = (a.q(1, 0, 1, 0) - a.q(1, 0, 1, -1)) * g.dzi;
+            const double F_EX32 = a.ms(2, 0, 1, 0) * DVDZ, F_IM32 = a.ms(2, 0, 1, 0) * DWDY;
+            DWDY = (a.q(2, 0, 0, 0) - a.q(2, 0, -1, 0)) * dycij;
+            DVDZ = (a.q(1, 0, 0, 0) - a.q(1, 0, 0, -1)) * g.dzi;
+            const double B_EX32 = a.ms(2, 0, 0, 0) * DVDZ, B_IM32 = a.ms(2, 0, 0, 0) * DWDY;
+            const double D32_EX = (F_EX32 - B_EX32) * coe2;
+            const double D32_IM = (F_IM32 - B_IM32) * coe2;
+            ex3 = D31_EX + D32_EX + D33_EX + ex3;
+            im3 = D31_IM + D32_IM + D33_IM;
+        }
+    }
+}
+
+// RHS_MOM_EXPLICIT_io at one point (c, ii: its padded and interior index; pc, pim, pjm, pkm: the pressure there
+// and at its lower neighbours; e0: the three EXPLT0 values): writes EXPLT0 and RHS, returns the point's x
+// right-hand side for the bulk forcing (0 at a fixed inlet face).
+template <bool CN, typename F>
+__device__ __forceinline__ double io_rhs_combine(const Geo& g, const IoFieldsT<F>& f, int i, int j, int k, long long c, long long ii,
+                                                 double dycij, int ns, double dt, double ex1, double ex2, double ex3, double im1, double im2, double im3,
+                                                 double pc, double pim, double pjm, double pkm, double e01, double e02, double e03) {
+    const long long FS = g.FS;
+    const long long cim = c + (xmn(g, i) - i), cjm = c - g.L, ckm = c + (wrapm(k, g.N) - k) * g.P;
+    const double tg = g.tgam[ns], tr = g.troh[ns], ta = g.talp[ns];
+    // with inflow the inlet face u(1) is a boundary value: its x-momentum RHS, EXPLT0 and
+    // G are left alone (NXI = 2, src/RHS_MOM_EXPLICIT_io.f90:35)
+    const bool ux = !(g.xo && i == 1);
+    const double coa = ta * dt;
+    // buoyancy (:161-226): D_STG * TALP*DT*F_A on the component |iGravity| (1/RNDI1 = 1/RCCI1 = 1)
+    const int ig = f.igrav < 0 ? -f.igrav : f.igrav;
+    const double cob = ta * dt * f.fa;
+    double r1 = (tg * ex1 + tr * e01) * dt;
+    if constexpr (CN) r1 = r1 + coa * im1;
+    r1 = r1 - io_pgm(f, c, cim, pc, pim, ta * dt * g.dxi);
+    if (ig == 1) r1 = r1 + f.DST[c] * cob;
+    double r3 = (tg * ex3 + tr * e03) * dt;
+    if constexpr (CN) r3 = r3 + coa * im3;
+    r3 = r3 - io_pgm(f, c, ckm, pc, pkm, ta * dt * g.dzi);
+    if (ig == 3) r3 = r3 + f.DST[c + 2 * FS] * (cob / 1.0);
+    if (ux) {
+        f.EX0[ii] = (F)ex1;
+        f.RHS[ii] = (F)r1;
+    }
+    f.EX0[ii + 2 * g.FI] = (F)ex3;
+    f.RHS[ii + 2 * g.FI] = (F)r3;
+    if (j >= 2) {
+        double r2 = (tg * ex2 + tr * e02) * dt;
+        if constexpr (CN) r2 = r2 + coa * im2;
+        r2 = r2 - io_pgm(f, c, cjm, pc, pjm, ta * dt * dycij / 1.0);
+        if (ig == 2) r2 = r2 + f.DST[c + FS] * (cob / 1.0);
+        f.EX0[ii + g.FI] = (F)ex2;
+        f.RHS[ii + g.FI] = (F)r2;
+    }
+    return ux ? r1 : 0.0;
+}
+
+// Grid sum of the bulk-forcing integrand: block partials, added by the last block to finish, in order
+template <int NT>
+__device__ __forceinline__ void io_rhs_bulk(double bulk, double* sred, double* __restrict__ partial, DevState* __restrict__ st) {
+    __shared__ int is_last;
+    double s = block_sum<NT>(bulk, sred);
     if (threadIdx.x == 0) {
         partial[blockIdx.x] = s;
         __threadfence();
@@ -432,13 +428,206 @@ __global__ void __launch_bounds__(IO_NT, 2) k_io_rhs(Geo g, IoFieldsT<F> f, doub
     if (is_last) {
         __threadfence();
         double a = 0.0;
-        for (int t = threadIdx.x; t < (int)gridDim.x; t += IO_NT) a += __ldcg(partial + t);
-        a = block_sum<IO_NT>(a, sred);
+        for (int t = threadIdx.x; t < (int)gridDim.x; t += NT) a += __ldcg(partial + t);
+        a = block_sum<NT>(a, sred);
         if (threadIdx.x == 0) {
             st->bulksum = a;
             st->ctr = 0u;
         }
     }
+}
+
+// neighbours of one point in global memory
+template <typename F>
+struct IoGlobal {
+    const F *Q, *G, *MS, *DV;
+    const double *U0, *U;
+    long long FS, c, dip, dim, djp, djm, dkp, dkm;
+    __device__ __forceinline__ long long at(int di, int dj, int dk) const {
+        return c + (di > 0 ? dip : di < 0 ? dim : 0) + (dj > 0 ? djp : dj < 0 ? djm : 0) + (dk > 0 ? dkp : dk < 0 ? dkm : 0);
+    }
+    __device__ __forceinline__ F q(int n, int di, int dj, int dk) const { return Q[at(di, dj, dk) + n * FS]; }
+    __device__ __forceinline__ F g(int n, int di, int dj, int dk) const { return G[at(di, dj, dk) + n * FS]; }
+    __device__ __forceinline__ F ms(int n, int di, int dj, int dk) const { return MS[at(di, dj, dk) + n * FS]; }
+    __device__ __forceinline__ double u0(int di, int dj, int dk) const { return U0[at(di, dj, dk)]; }
+    __device__ __forceinline__ double u(int di, int dj, int dk) const { return U[at(di, dj, dk)]; }
+    __device__ __forceinline__ F dv(int di, int dj, int dk) const { return DV[at(di, dj, dk)]; }
+};
+
+// FP32 storage: one thread per point in flat order.  (The order of the bulk sum decides the last bit of the
+// forcing, and with FP32 storage a changed last bit of an FP64 value is a changed stored value now and
+// then, so this form keeps its order.)
+template <bool CN, typename F>
+__global__ void __launch_bounds__(IO_NT, 2) k_io_rhs(Geo g, IoFieldsT<F> f, double* __restrict__ partial, DevState* __restrict__ st,
+                                                  int ns) {
+    __shared__ double sred[32];
+    const int N = g.N;
+    const long long tot = io_points(g);
+    const double dt = st->dt;
+    double bulk = 0.0;
+    for (long long t = (long long)blockIdx.x * IO_NT + threadIdx.x; t < tot; t += (long long)gridDim.x * IO_NT) {
+        int i, j, k;
+        io_decode(g, t, i, j, k);
+        const long long c = pidx(g, i, j, k), cim = pidx(g, xmn(g, i), j, k), ckm = pidx(g, i, j, wrapm(k, N));
+        const IoGlobal<F> a{f.Q, f.G, f.MST, f.DIVU, f.MU0, f.MU, g.FS, c, pidx(g, xpn(g, i), j, k) - c, cim - c, g.L, -g.L,
+                            pidx(g, i, j, wrapp(k, N)) - c, ckm - c};
+        double ex1, ex2, ex3, im1, im2, im3;
+        io_rhs_terms<CN>(g, io_row(g, j), a, j, ex1, ex2, ex3, im1, im2, im3);
+        const long long ii = io_iidx(g, i, j, k);
+        const double e01 = f.EX0[ii], e02 = f.EX0[ii + g.FI], e03 = f.EX0[ii + 2 * g.FI];
+        bulk += io_rhs_combine<CN>(g, f, i, j, k, c, ii, g.dyci[j], ns, dt, ex1, ex2, ex3, im1, im2, im3, f.PR[c], f.PR[cim], f.PR[c - g.L],
+                                   f.PR[ckm], e01, e02, e03) / g.dyfi[j] / 1.0;
+    }
+    io_rhs_bulk<IO_NT>(bulk, sred, partial, st);
+}
+
+// FP64: a block of 32 x 16 threads owns 32 (i) x 16 (j) columns and marches over `chunk` planes in k.  The
+// planes of the fields, tile and one-point halo, are in shared memory (rings of four planes for Q and G,
+// three for MU_STG, the viscosity and PR), the next one arriving by asynchronous copies while a plane is
+// computed.  The flat form reads about 75 neighbour values per point from L1 and L2 with 16 warps per SM
+// to wait for them, in 900 instructions, half of them addresses; here every neighbour is a
+// shared-memory read at a constant offset and each field is fetched once per tile.  The explicit scheme's
+// DivU is formed from Q in shared memory (DIVG_U_io's pass over the fields is not needed).  One block per
+// SM by shared memory; bound by the latencies of its 16 warps (issue slots a third busy).  Per step (three
+// launches): Crank-Nicolson at 256 x 192 x 128 1.55 -> 1.08 ms, explicit with DivU at 128^3 0.55 -> 0.41.
+constexpr int IT_I = 32, IT_J = 16, IT_NT = IT_I * IT_J;
+constexpr int IT_HI = IT_I + 2, IT_PL = IT_HI * (IT_J + 2);      // row and plane of a tile with its halo
+constexpr int IT_SMEM = (6 * 4 + 3 * 3 + 2 * 3) * IT_PL * 8;     // bytes
+
+// planes per block: the split of N that gives the least time, counted in planes loaded by the busiest SM (one
+// block per SM; each block loads three more planes than it computes)
+inline int io_tile_chunk(const Geo& g, int nsm) {
+    const int tiles = ((g.LI + IT_I - 1) / IT_I) * (g.M / IT_J);
+    int best = g.N;
+    long long cost = -1;
+    for (int n = 1; n <= g.N / 8; ++n) {
+        const int chunk = (g.N + n - 1) / n;
+        const int nb = (g.N + chunk - 1) / chunk;
+        const long long t = (long long)((tiles * nb + nsm - 1) / nsm) * (chunk + 3);
+        if (cost < 0 || t < cost) { cost = t; best = chunk; }
+    }
+    return best;
+}
+inline int io_tile_blocks(const Geo& g, int chunk) {
+    return ((g.LI + IT_I - 1) / IT_I) * (g.M / IT_J) * ((g.N + chunk - 1) / chunk);
+}
+
+struct IoTileAcc {  // neighbours of one point in the tile's planes
+    const double *qm, *qc, *qp, *mc, *mp, *vm, *vc;  // Q and G, MU_STG, viscosity and PR at planes k - 1, k, k + 1
+    double dxi, dzi, dyfij, dyfim;
+    static __device__ __forceinline__ int o(int di, int dj) { return di + IT_HI * dj; }
+    __device__ __forceinline__ double q(int n, int di, int dj, int dk) const { return (dk > 0 ? qp : dk < 0 ? qm : qc)[n * IT_PL + o(di, dj)]; }
+    __device__ __forceinline__ double g(int n, int di, int dj, int dk) const { return q(3 + n, di, dj, dk); }
+    __device__ __forceinline__ double ms(int n, int di, int dj, int dk) const { return (dk > 0 ? mp : mc)[n * IT_PL + o(di, dj)]; }
+    __device__ __forceinline__ double u0(int di, int dj, int dk) const { return (dk < 0 ? vm : vc)[o(di, dj)]; }
+    __device__ __forceinline__ double u(int di, int dj, int dk) const { return u0(di, dj, dk); }
+    __device__ __forceinline__ double pr(int di, int dj, int dk) const { return (dk < 0 ? vm : vc)[IT_PL + o(di, dj)]; }
+    // DIVG_U_io at the point (0 0 0) or its lower neighbour in one direction
+    __device__ __forceinline__ double dv(int di, int dj, int dk) const {
+        const double dx = (q(0, di + 1, dj, dk) - q(0, di, dj, dk)) * dxi;
+        const double dy = (q(1, di, dj + 1, dk) - q(1, di, dj, dk)) * (dj < 0 ? dyfim : dyfij);
+        const double dz = (q(2, di, dj, dk + 1) - q(2, di, dj, dk)) * dzi;
+        return (dx + dy + dz) * (1.0 / 3.0);
+    }
+};
+
+template <bool CN>
+__global__ void __launch_bounds__(IT_NT, 1) k_io_rhs_tile(Geo g, IoFields f, double* __restrict__ partial, DevState* __restrict__ st,
+                                                         int ns, int chunk) {
+    extern __shared__ __align__(16) double smt[];
+    __shared__ double sred[32];
+    // the rows' y coefficients: in shared memory, as the L1 left beside the rings is small and the planes
+    // stream through it
+    __shared__ IoRow srow[IT_J];
+    const int N = g.N, nti = (g.LI + IT_I - 1) / IT_I, ntj = g.M / IT_J;
+    const int b = blockIdx.x, r = b / nti, kc = r / ntj;
+    const int i0 = IT_I * (b - r * nti) + g.xo, j0 = 1 + IT_J * (r - kc * ntj);
+    const int k0 = kc * chunk, k1 = min(N, k0 + chunk);
+    const int i = i0 + (threadIdx.x & 31), j = j0 + (threadIdx.x >> 5);
+    const bool on = i - g.xo < g.LI;
+    const double dt = st->dt;
+    double* const smq = smt;                     // 4 planes of Q, G
+    double* const smm = smq + 4 * 6 * IT_PL;     // 3 planes of MU_STG
+    double* const smv = smm + 3 * 3 * IT_PL;     // 3 planes of the viscosity and PR
+    // this thread's points of a plane: padded offsets at k = 0 (columns past the row's last storage column
+    // repeat it; they feed only threads that are off)
+    constexpr int NE = (IT_PL + IT_NT - 1) / IT_NT;
+    long long eo[NE];
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+        const int q = threadIdx.x + e * IT_NT, jj = q / IT_HI;
+        int ii = i0 - 1 + (q - jj * IT_HI);
+        if (g.xo) ii = min(ii, g.L - 1);
+        else ii = ii < 0 ? ii + g.L : ii >= g.L ? ii - g.L : ii;
+        eo[e] = q < IT_PL ? pidx(g, ii, j0 - 1 + jj, 0) : -1;
+    }
+    auto wrap = [&](int k) { return k < 0 ? k + N : k >= N ? k - N : k; };
+    auto load_q = [&](int k, double* dst) {
+        const long long ko = g.P * wrap(k);
+#pragma unroll
+        for (int e = 0; e < NE; ++e)
+            if (eo[e] >= 0) {
+                double* d = dst + threadIdx.x + e * IT_NT;
+                const long long o = eo[e] + ko;
+#pragma unroll
+                for (int n = 0; n < 3; ++n) {
+                    cp_async8(d + n * IT_PL, f.Q + o + n * g.FS);
+                    cp_async8(d + (3 + n) * IT_PL, f.G + o + n * g.FS);
+                }
+            }
+    };
+    auto load_m = [&](int k, double* dst) {
+        const long long ko = g.P * wrap(k);
+#pragma unroll
+        for (int e = 0; e < NE; ++e)
+            if (eo[e] >= 0) {
+#pragma unroll
+                for (int n = 0; n < 3; ++n) cp_async8(dst + threadIdx.x + e * IT_NT + n * IT_PL, f.MST + eo[e] + ko + n * g.FS);
+            }
+    };
+    auto load_v = [&](int k, double* dst) {
+        const long long ko = g.P * wrap(k);
+        const double* U = CN ? f.MU : f.MU0;
+#pragma unroll
+        for (int e = 0; e < NE; ++e)
+            if (eo[e] >= 0) {
+                double* d = dst + threadIdx.x + e * IT_NT;
+                cp_async8(d, U + eo[e] + ko);
+                cp_async8(d + IT_PL, f.PR + eo[e] + ko);
+            }
+    };
+    constexpr int QS = 6 * IT_PL, MSZ = 3 * IT_PL, VS = 2 * IT_PL;
+    int sq = 1, sm = 0, sv = 1;  // ring slots of plane k
+    load_q(k0 - 1, smq); load_q(k0, smq + QS); load_q(k0 + 1, smq + 2 * QS);
+    load_m(k0, smm); load_m(k0 + 1, smm + MSZ);
+    load_v(k0 - 1, smv); load_v(k0, smv + VS);
+    const int cc = (threadIdx.x >> 5) * IT_HI + IT_HI + (threadIdx.x & 31) + 1;  // this point inside a plane
+    if (threadIdx.x < IT_J) srow[threadIdx.x] = io_row(g, j0 + threadIdx.x);
+    const IoRow& y = srow[threadIdx.x >> 5];
+    long long c = pidx(g, i, j, k0), ii = io_iidx(g, i, j, k0);
+    double bulk = 0.0;
+#pragma unroll 1
+    for (int k = k0; k < k1; ++k, c += g.P, ii += g.PI_) {
+        const int sqp = (sq + 1) & 3, sqm = (sq + 3) & 3, smp = sm == 2 ? 0 : sm + 1, svm = sv == 0 ? 2 : sv - 1;
+        cp_async_wait_all();
+        __syncthreads();  // planes k - 1 .. k + 1 are here, and every thread is done with the slots filled next
+        if (k + 1 < k1) {
+            load_q(k + 2, smq + ((sq + 2) & 3) * QS);
+            load_m(k + 2, smm + (sm == 0 ? 2 : sm - 1) * MSZ);
+            load_v(k + 1, smv + (sv == 2 ? 0 : sv + 1) * VS);
+        }
+        if (on) {
+            const double e01 = f.EX0[ii], e02 = f.EX0[ii + g.FI], e03 = f.EX0[ii + 2 * g.FI];
+            const IoTileAcc a{smq + sqm * QS + cc, smq + sq * QS + cc, smq + sqp * QS + cc, smm + sm * MSZ + cc, smm + smp * MSZ + cc,
+                              smv + svm * VS + cc, smv + sv * VS + cc, g.dxi, g.dzi, y.dyfij, y.dyfim};
+            double ex1, ex2, ex3, im1, im2, im3;
+            io_rhs_terms<CN>(g, y, a, j, ex1, ex2, ex3, im1, im2, im3);
+            bulk += io_rhs_combine<CN>(g, f, i, j, k, c, ii, y.dycij, ns, dt, ex1, ex2, ex3, im1, im2, im3, a.pr(0, 0, 0), a.pr(-1, 0, 0),
+                                       a.pr(0, -1, 0), a.pr(0, 0, -1), e01, e02, e03);
+        }
+        sq = sqp; sm = smp; sv = sv == 2 ? 0 : sv + 1;
+    }
+    io_rhs_bulk<IT_NT>(bulk / g.dyfi[j], sred, partial, st);  // one row per thread
 }
 
 // bulk forcing (RHS_MOM_EXPLICIT_io :228-265) + MASSFLUX_CALC_io

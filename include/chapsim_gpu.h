@@ -559,7 +559,7 @@ int chapsim_batch_destroy(chapsim_batch_t* batch);
  * Main domain: k_io_cfl, k_dt, then for each substep (with the thermal
  * solver) k_eng_rhs, the property update (table search or model), k_eng_bc,
  * k_eng_state and two empty slots, then the momentum step's three
- * slots (explicit: k_io_divu, k_io_rhs, k_io_massflux; Crank-Nicolson:
+ * slots (explicit: k_io_divu (empty in FP64), k_io_rhs, k_io_massflux; Crank-Nicolson:
  * k_io_rhs, the x sweep, the z and y sweeps) and k_io_div_fftx, k_fftz_fwd,
  * k_ysolve, k_fftz_inv, k_fftx_inv, k_io_correct (29 slots, 47 with the
  * thermal solver). */
