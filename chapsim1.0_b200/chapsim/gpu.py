@@ -638,10 +638,7 @@ class ChannelTG:
         transforms; bit 4: two-way y-solve; bit 5: sequential y-solve with its
         forward intermediate in shared memory at one block per SM; bit 6: warp
         affine scans over the sequential factors; bit 8: z-sweep tiles of 16
-        lines instead of 32; bit 9: double-buffered persistent z transforms; bit 10:
-        z-sweep tiles with the lines interleaved in pairs; bit 11: the same for the y sweep;
-        bit 12: z transforms that request the next wave's tiles into L2);
-        returns
+        lines instead of 32; bits 9-12: kept as forced, no effect); returns
         (choice bits, {variant: ms})."""
         ch = ctypes.c_int32()
         ms = (ctypes.c_float * 19)()

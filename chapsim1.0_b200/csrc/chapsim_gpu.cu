@@ -166,8 +166,7 @@ struct chapsim_ctx {
     int zs_tw = 32;               // lines per tile of the z sweep, 32 or 16 (chapsim_autotune)
     int zs_il = 1;                // FP32 z-sweep tile layout: 1 line-contiguous, 2 lines interleaved in pairs (chapsim_autotune)
     int ys_il = 1;                // the same for the FP32 y sweep (chapsim_autotune)
-    bool fz_pipe = false;         // persistent double-buffered z transforms (chapsim_autotune)
-    bool fz_prefetch = false;     // one-tile z transforms request the tile one wave ahead into L2 (chapsim_autotune)
+    bool fz_pipe = false, fz_prefetch = false;  // bits 9 and 12 of chapsim_autotune, kept as forced (no effect)
     bool p2c = false;             // the fused plane transforms run as a thread-block cluster (k_div_fft2c/k_fft2c_inv)
     int rb_nw = 0;                // warps per block of k_rhs_xsweep_bulk (0: the stages do not fit)
     bool pdl = true;              // step kernels launched with programmatic dependent launch
@@ -305,9 +304,7 @@ int rt_chunk(const Geo& g) {
 template <typename C = double2>
 size_t smem_px(const Geo& g) { return (size_t)((PX_TJ / 2) * fft4s_ld(g.L)) * sizeof(C); }
 template <typename C = double2>
-size_t smem_fz(const Geo& g) { return (size_t)(FZ_TQ * fft4s_ld(g.N)) * sizeof(C); }
-template <typename C>
-size_t smem_fzp(const Geo& g) { return (size_t)(2 * fzp_tq<C>() * fft4s_ld(g.N)) * sizeof(C); }
+size_t smem_fz(const Geo& g) { return (size_t)(fz_tq<C>() * fft4s_ld(g.N)) * sizeof(C); }
 // the context's pressure increment DPH in the step's real type
 template <typename R> R* dph(chapsim_ctx* c);
 template <> double* dph<double>(chapsim_ctx* c) { return c->DPH; }
@@ -519,8 +516,6 @@ int configure_momentum(chapsim_ctx* ctx) {
         P2C_DISPATCH(g.L, g.N, (ctx->p2c = plane_fft_cluster_setup<R, XN1, XN2, ZN1, ZN2>(g)));
     DISPATCH_FFT(g.N, CK(set_smem(k_fftz<-1, FN1, FN2, C>, smem_fz<C>(g))));
     DISPATCH_FFT(g.N, CK(set_smem(k_fftz<+1, FN1, FN2, C>, smem_fz<C>(g))));
-    DISPATCH_FFT(g.N, CK(set_smem(k_fftz_pipe<-1, FN1, FN2, C>, smem_fzp<C>(g))));
-    DISPATCH_FFT(g.N, CK(set_smem(k_fftz_pipe<+1, FN1, FN2, C>, smem_fzp<C>(g))));
     return CHAPSIM_OK;
 }
 
@@ -621,23 +616,12 @@ void launch_rhs_x(chapsim_ctx* ctx, const StepFields<R>& f, const R* fac, int ns
 // DIVG_tg + FFT99_POIS3D_periodicxz up to DPH: chained transforms, or the
 // fused plane transforms (one block per y row) where chosen.  Both record the
 // same profiling slots (the fused form leaves the two z-transform slots empty).
-// z transforms of the periodic channel's spectrum: one tile per block (k_fftz), or the
-// persistent double-buffered form (ctx->fz_pipe, chapsim_autotune bit 9)
+// z transforms of the spectrum
 template <int SIGN, typename C>
-void launch_fftz(chapsim_ctx* ctx, C* sp) {
+void launch_fftz(chapsim_ctx* ctx, C* sp, bool pdl) {
     const Geo& g = ctx->g;
-    const long long nq = (long long)g.LH * g.M;
-    if (ctx->fz_pipe) {
-        const long long nt = (nq + fzp_tq<C>() - 1) / fzp_tq<C>();
-        const int nb = (int)std::min<long long>(nt, (long long)fzp_minb<C>() * ctx->nsm);
-        DISPATCH_FFT(g.N, (launch_pdl(ctx->pdl, k_fftz_pipe<SIGN, FN1, FN2, C>, nb, fzp_nt<C>(), smem_fzp<C>(g), ctx->stream, g, sp)));
-    } else {
-        const int gfz = (int)((nq + FZ_TQ - 1) / FZ_TQ);
-        // prefetch distance: one wave of resident blocks (by the shared memory of a tile)
-        const int bps = std::max(1, std::min(sizeof(C) == 8 ? 4 : 2, (int)((227 * 1024) / smem_fz<C>(g))));
-        const int ahead = ctx->fz_prefetch ? bps * ctx->nsm : 0;
-        DISPATCH_FFT(g.N, (launch_pdl(ctx->pdl, k_fftz<SIGN, FN1, FN2, C>, gfz, FZ_NT, smem_fz<C>(g), ctx->stream, g, sp, ahead)));
-    }
+    const int gfz = (int)((long long)g.LH * g.M / fz_tq<C>());
+    DISPATCH_FFT(g.N, (launch_pdl(pdl, k_fftz<SIGN, FN1, FN2, C>, gfz, (fz_nt<C, FN1>()), smem_fz<C>(g), ctx->stream, g, sp)));
 }
 
 template <typename R>
@@ -669,13 +653,13 @@ void launch_pressure(chapsim_ctx* ctx, const StepFields<R>& f, int ns) {
     dim3 grp((g.M + PX_TJ - 1) / PX_TJ, g.N);
     DISPATCH_FFT(g.L, (launch_pdl(ctx->pdl, k_div_fftx<R, FN1, FN2>, grp, PX_NT, smem_px<C>(g), s, g, f.Q, f.RHSLL, sp, ctx->st, ns)));
     prof_mark(ctx);
-    launch_fftz<-1, C>(ctx, sp);
+    launch_fftz<-1, C>(ctx, sp, ctx->pdl);
     prof_mark(ctx);
     launch_ysolve<C>(ctx);
     prof_mark(ctx);
-    launch_fftz<+1, C>(ctx, sp);
+    launch_fftz<+1, C>(ctx, sp, ctx->pdl);
     prof_mark(ctx);
-    DISPATCH_FFT(g.L, (launch_pdl(ctx->pdl, k_fftx_inv<FN1, FN2, C>, grp, PX_NT, smem_px<C>(g), s, g, sp, dph<R>(ctx))));
+    DISPATCH_FFT(g.L, (launch_pdl(ctx->pdl, k_fftx_inv<FN1, FN2, C>, grp, px_nt<FN1>(), smem_px<C>(g), s, g, sp, dph<R>(ctx))));
     prof_mark(ctx);
     ctx->launches += 5;
 }
@@ -935,15 +919,13 @@ void launch_io_substep_t(chapsim_ctx* ctx, int ns) {
                                                                                ctx->thermal ? ctx->tf.DRHO : nullptr,
                                                                                ctx->io.PR0A ? 0.25 + IO_PRES_EPSLON : 1.0)));
     prof_mark(ctx);
-    const long long nq = (long long)g.LH * g.M;
-    const int gfz = (int)((nq + FZ_TQ - 1) / FZ_TQ);
-    DISPATCH_FFT(g.N, (k_fftz<-1, FN1, FN2, double2><<<gfz, FZ_NT, smem_fz(g), s>>>(g, ctx->SP, 0)));
+    launch_fftz<-1>(ctx, ctx->SP, false);
     prof_mark(ctx);
     launch_ysolve<double2>(ctx);
     prof_mark(ctx);
-    DISPATCH_FFT(g.N, (k_fftz<+1, FN1, FN2, double2><<<gfz, FZ_NT, smem_fz(g), s>>>(g, ctx->SP, 0)));
+    launch_fftz<+1>(ctx, ctx->SP, false);
     prof_mark(ctx);
-    DISPATCH_FFT(g.L, (k_fftx_inv<FN1, FN2, double2><<<grp, PX_NT, smem_px(g), s>>>(g, ctx->SP, ctx->DPH)));
+    DISPATCH_FFT(g.L, (k_fftx_inv<FN1, FN2, double2><<<grp, px_nt<FN1>(), smem_px(g), s>>>(g, ctx->SP, ctx->DPH)));
     prof_mark(ctx);
     k_io_correct<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->DPH, ctx->st, ns, ctx->ivis ? ctx->RHSLL : nullptr);
     prof_mark(ctx);
@@ -1002,13 +984,11 @@ void launch_xio_substep(chapsim_ctx* ctx, int ns) {
         k_xio_div_dctx<<<nrb, XIO_NT, smem_xd(g), s>>>(g, f.G, ctx->xio_cf, ctx->SP, ctx->st, ns, 1.0, drho);
     }
     prof_mark(ctx);
-    const long long nq = (long long)g.LH * g.M;  // LH = LI x modes
-    const int gfz = (int)((nq + FZ_TQ - 1) / FZ_TQ);
-    DISPATCH_FFT(g.N, (k_fftz<-1, FN1, FN2, double2><<<gfz, FZ_NT, smem_fz(g), s>>>(g, ctx->SP, 0)));
+    launch_fftz<-1>(ctx, ctx->SP, false);
     prof_mark(ctx);
     k_xio_ysolve<<<(int)(((long long)g.LI * g.N + XIO_NT - 1) / XIO_NT), XIO_NT, 0, s>>>(g, ctx->SP, ctx->xio_yd);
     prof_mark(ctx);
-    DISPATCH_FFT(g.N, (k_fftz<+1, FN1, FN2, double2><<<gfz, FZ_NT, smem_fz(g), s>>>(g, ctx->SP, 0)));
+    launch_fftz<+1>(ctx, ctx->SP, false);
     prof_mark(ctx);
     if (fftx) {
         DISPATCH_FFT(g.LI, (k_xio_cosqb<FN1, FN2><<<gxf, PX_NT, smf, s>>>(g, ctx->SP, ctx->xio_tq, ctx->DPH)));
@@ -1830,12 +1810,10 @@ int chapsim_fft99_pois3d(chapsim_ctx_t* ctx, const double* rhs, double* dph) {
     CK(cudaMemcpyAsync(ctx->RHSLL, rhs, (size_t)g.FI * sizeof(double), cudaMemcpyHostToDevice, s));
     dim3 grp((g.M + PX_TJ - 1) / PX_TJ, g.N);
     DISPATCH_FFT(g.L, (k_fftx_from_rhs<FN1, FN2><<<grp, PX_NT, smem_px(g), s>>>(g, ctx->RHSLL, ctx->SP)));
-    const long long nq = (long long)g.LH * g.M;
-    const int gfz = (int)((nq + FZ_TQ - 1) / FZ_TQ);
-    DISPATCH_FFT(g.N, (k_fftz<-1, FN1, FN2, double2><<<gfz, FZ_NT, smem_fz(g), s>>>(g, ctx->SP, 0)));
+    launch_fftz<-1>(ctx, ctx->SP, false);
     launch_ysolve<double2>(ctx);
-    DISPATCH_FFT(g.N, (k_fftz<+1, FN1, FN2, double2><<<gfz, FZ_NT, smem_fz(g), s>>>(g, ctx->SP, 0)));
-    DISPATCH_FFT(g.L, (k_fftx_inv<FN1, FN2, double2><<<grp, PX_NT, smem_px(g), s>>>(g, ctx->SP, ctx->DPH)));
+    launch_fftz<+1>(ctx, ctx->SP, false);
+    DISPATCH_FFT(g.L, (k_fftx_inv<FN1, FN2, double2><<<grp, px_nt<FN1>(), smem_px(g), s>>>(g, ctx->SP, ctx->DPH)));
     ctx->launches += 5;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(dph, ctx->DPH, (size_t)g.FS * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -2975,17 +2953,15 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
     // pressure stage up to DPH: chained x/z transforms or the fused plane
     // transforms (periodic channel, planes that fit one block).  It writes
     // only scratch (RHSLLPHI, the spectrum, DPH), which every substep rewrites.
-    // (kind 0: chained transforms, 1: fused plane transforms, 2: chained with the persistent
-    // double-buffered z transforms, 3: chained with the z transforms' wave-ahead L2 requests)
+    // (kind 0: chained transforms, 1: fused plane transforms; bits 9 and 12 chose other forms of the z
+    // transform, which loads everything it needs at once now: they are kept, timed as kind 0)
     float tp[4] = {0.f, 1e30f, 0.f, 0.f};
     if (ctx->domain == 1) {
         const bool mixed = ctx->prec == CHAPSIM_PREC_MIXED;
         bool p2 = (mixed ? plane_fft_ok<float2>(g) : plane_fft_ok<double2>(g)) || ctx->p2c;
-        for (int kind = 0; kind < 4; ++kind) {
+        for (int kind = 0; kind < 2; ++kind) {
             if (kind == 1 && !p2) continue;
-            ctx->plane_kind = kind == 1 ? 1 : 0;
-            ctx->fz_pipe = kind == 2;
-            ctx->fz_prefetch = kind == 3;
+            ctx->plane_kind = kind;
             auto one = [&]() {
                 if (mixed) launch_pressure<float>(ctx, step_fields<float>(ctx), 1);
                 else launch_pressure<double>(ctx, step_fields<double>(ctx), 1);
@@ -3011,13 +2987,10 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
             ctx->fz_pipe = (force & 512) != 0;
             ctx->fz_prefetch = (force & 4096) != 0;
         } else {
-            int best = 0;
-            for (int kind = 1; kind < 4; ++kind)
-                if (tp[kind] < tp[best]) best = kind;
-            ctx->plane_kind = best == 1 ? 1 : 0;
-            ctx->fz_pipe = best == 2;
-            ctx->fz_prefetch = best == 3;
+            ctx->plane_kind = tp[1] < tp[0] ? 1 : 0;
+            ctx->fz_pipe = ctx->fz_prefetch = false;
         }
+        tp[2] = tp[3] = tp[0];
     }
     if (ctx->step_exec) {
         cudaGraphExecDestroy(ctx->step_exec);

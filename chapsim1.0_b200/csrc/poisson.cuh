@@ -49,11 +49,8 @@ template <> __device__ __forceinline__ float2 from_d2<float2>(double2 a) { retur
 #define PX_NT 128
 #define PX_MINB 4
 // FP32 transforms: eight blocks per SM within 64 registers (twice the warps to
-// hide the latency of the load, transform and store phases); the z transform
-// likewise runs four FP32 blocks of FZ_NT threads per SM instead of two
+// hide the latency of the load, transform and store phases)
 template <typename C> __host__ __device__ constexpr int px_minb() { return sizeof(C) == 8 ? 8 : PX_MINB; }
-#define FZ_TQ 16  // z-lines per block
-#define FZ_NT 256
 #define CR_NT 256
 
 // ---------------------------------------------------------------------------
@@ -138,114 +135,71 @@ __global__ void __launch_bounds__(PX_NT, px_minb<SpecT<R>>()) k_div_fftx(Geo g, 
 }
 
 // ---------------------------------------------------------------------------
-// complex z transform of FZ_TQ consecutive (kx, j) lines (index q = kx + LH*(j-1))
-// pf_ahead > 0: the block also requests into L2 the tile of block blockIdx.x + pf_ahead (about
-// one wave of resident blocks later), whose copies then find their rows there.
+// The two passes of the four-step FFT (fft.cuh) on registers: a thread holds one length-N2 (first
+// pass) or length-N1 (second pass) transform, and only the exchange between the passes goes through
+// shared memory.  buf: the line's n + n2 + 1 words.
+template <int N1, int N2, int SIGN, typename C>
+__device__ __forceinline__ void fft_first(C (&v)[N2], C* buf, int j1, const C* __restrict__ tw) {
+    SmallDft<N2, SIGN, C>::run(v);
+#pragma unroll
+    for (int k2 = 0; k2 < N2; ++k2) {
+        C w = tw[j1 * k2];
+        if (SIGN > 0) w.y = -w.y;
+        buf[k2 * (N1 + 1) + j1] = (j1 == 0 || k2 == 0) ? v[k2] : cmul(v[k2], w);
+    }
+}
+template <int N1, int SIGN, typename C>
+__device__ __forceinline__ void fft_second(C (&v)[N1], const C* buf, int k2) {
+#pragma unroll
+    for (int j1 = 0; j1 < N1; ++j1) v[j1] = buf[k2 * (N1 + 1) + j1];
+    SmallDft<N1, SIGN, C>::run(v);
+}
+
+// x-line blocks: PX_TJ y rows as PX_TJ / 2 packed pairs, N1 threads per pair
+template <int N1> __host__ __device__ constexpr int px_nt() { return PX_TJ / 2 * N1; }
+template <typename C, int N1> __host__ __device__ constexpr int px_rminb() { return (sizeof(C) == 8 ? 1024 : 512) / px_nt<N1>(); }
+// complex z transform of TQ consecutive (kx, j) lines (index q = kx + LH*(j-1); LH M is a multiple of
+// 32): thread (ql, j1) loads the N2 values of its first-pass transform straight into registers, all in
+// flight together, as row pieces of TQ complex values (128 bytes), and the second pass's results go from
+// registers to memory.  Staging the tile in shared memory on both sides (asynchronous copies in, a
+// pass out) cost four more moves of every value and three more block barriers.  Both directions, per
+// step: 0.21 -> 0.12 ms at 256 x 192 x 128, 0.18 -> 0.10 at 192 x 128 x 192, 1.29 -> 1.03 at 384 x 256 x 384 (24
+// complex values in registers: the load, transform and store phases of two blocks per SM in turn), FP32 there
+// 0.62 -> 0.49.  The FP32 fields are the same to the bit.
+template <typename C> __host__ __device__ constexpr int fz_tq() { return 128 / (int)sizeof(C); }
+template <typename C, int N1> __host__ __device__ constexpr int fz_nt() { return fz_tq<C>() * N1; }
+template <typename C, int N1> __host__ __device__ constexpr int fz_minb() { return (sizeof(C) == 8 ? 1024 : 512) / fz_nt<C, N1>(); }
 template <int SIGN, int N1, int N2, typename C>
-__global__ void __launch_bounds__(FZ_NT, sizeof(C) == 8 ? 4 : 2) k_fftz(Geo g, C* __restrict__ SP, int pf_ahead) {
+__global__ void __launch_bounds__((fz_nt<C, N1>()), (fz_minb<C, N1>())) k_fftz(Geo g, C* __restrict__ SP) {
     pdl_wait();
     using T = typename CReal<C>::T;
     extern __shared__ __align__(16) unsigned char smp_raw[];
     C* smc = reinterpret_cast<C*>(smp_raw);
-    const int N = g.N;
-    const int LD = fft4s_ld(N);
+    constexpr int N = N1 * N2, LD = N + N2 + 1, TQ = fz_tq<C>();
     const long long Q = (long long)g.LH * g.M;
-    const long long q0 = (long long)blockIdx.x * FZ_TQ;
-    const int nq = (int)min((long long)FZ_TQ, Q - q0);
-    if (pf_ahead > 0) {
-        const long long qa = q0 + (long long)pf_ahead * FZ_TQ;
-        if (qa + FZ_TQ <= Q) {
-            constexpr int LPR = (FZ_TQ * (int)sizeof(C) + 127) / 128;  // 128-byte lines per kz row of a tile
-            for (int t = threadIdx.x; t < N * LPR; t += FZ_NT) {
-                const int kz = t / LPR, c = t - kz * LPR;
-                prefetch_l2(reinterpret_cast<const char*>(SP + qa + Q * kz) + 128 * c);
-            }
-        }
+    const int ql = threadIdx.x % TQ, j1 = threadIdx.x / TQ;
+    C* const sp = SP + (long long)blockIdx.x * TQ + ql;
+    {
+        C v[N2];
+        const C* src = sp + Q * j1;
+#pragma unroll
+        for (int j2 = 0; j2 < N2; ++j2) v[j2] = src[Q * (N1 * j2)];
+        fft_first<N1, N2, SIGN>(v, smc + ql * LD, j1, twz_of<C>(g));
     }
-    for (int p = threadIdx.x; p < FZ_TQ * N; p += FZ_NT) {
-        const int kz = p / FZ_TQ, ql = p - kz * FZ_TQ;
-        if (ql < nq) {
-            if constexpr (sizeof(C) == 16) cp_async16(smc + ql * LD + kz, SP + q0 + ql + Q * kz);
-            else cp_async8(reinterpret_cast<double*>(smc + ql * LD + kz), reinterpret_cast<const double*>(SP + q0 + ql + Q * kz));
-        }
-    }
-    cp_async_wait_all();
-    block_fft4s<N1, N2, SIGN>(smc, nq, LD, twz_of<C>(g));
+    __syncthreads();
     const T sc = SIGN < 0 ? (T)(1.0 / (double)N) : (T)1.0;
-    for (int p = threadIdx.x; p < FZ_TQ * N; p += FZ_NT) {
-        const int kz = p / FZ_TQ, ql = p - kz * FZ_TQ;
-        if (ql < nq) {
-            C v = smc[ql * LD + kz];
-            if (SIGN < 0) { v.x = v.x * sc; v.y = v.y * sc; }
-            SP[q0 + ql + Q * kz] = v;
+#pragma unroll 1
+    for (int k2 = j1; k2 < N2; k2 += N1) {
+        C v[N1];
+        fft_second<N1, SIGN>(v, smc + ql * LD, k2);
+        C* dst = sp + Q * k2;
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) {
+            C x = v[k1];
+            if (SIGN < 0) { x.x = x.x * sc; x.y = x.y * sc; }
+            dst[Q * (N2 * k1)] = x;
         }
     }
-}
-
-// Persistent, double-buffered form of k_fftz (autotuned alternative): a block
-// owns every gridDim.x-th tile of TQ lines and issues the copies of its
-// next tile (cp.async into the other buffer) before it transforms and stores
-// the current one, so the loads overlap the transform and the stores, where
-// the one-tile blocks of k_fftz overlap them only across blocks.  The
-// arithmetic is k_fftz's: the fields are bitwise equal.
-// Two blocks per SM at both precisions.  FP64: tiles of 8 lines (two 51 KB buffers at
-// N = 384) and 128 threads, whose register budget holds the 384-point transform inside the
-// persistent tile loop (at 256 threads and 128 registers it spilled 700 bytes); FP32: tiles
-// of 16 lines and 256 threads.
-template <typename C> __host__ __device__ constexpr int fzp_tq() { return sizeof(C) == 16 ? 8 : 16; }
-template <typename C> __host__ __device__ constexpr int fzp_nt() { return sizeof(C) == 16 ? 128 : 256; }
-template <typename C> __host__ __device__ constexpr int fzp_minb() { return 2; }
-
-template <int SIGN, int N1, int N2, typename C>
-__global__ void __launch_bounds__(fzp_nt<C>(), fzp_minb<C>()) k_fftz_pipe(Geo g, C* __restrict__ SP) {
-    pdl_wait();
-    constexpr int TQ = fzp_tq<C>();
-    constexpr int NT = fzp_nt<C>();
-    using T = typename CReal<C>::T;
-    extern __shared__ __align__(16) unsigned char smp_raw[];
-    const int N = g.N;
-    const int LD = fft4s_ld(N);
-    C* const buf0 = reinterpret_cast<C*>(smp_raw);
-    const long long Q = (long long)g.LH * g.M;
-    const long long ntile = (Q + TQ - 1) / TQ;
-    auto issue = [&](long long tile, C* b) {
-        if (tile < ntile) {
-            const long long q0 = tile * TQ;
-            const int nq = (int)min((long long)TQ, Q - q0);
-#pragma unroll 1
-            for (int p = threadIdx.x; p < TQ * N; p += NT) {
-                const int kz = p / TQ, ql = p - kz * TQ;
-                if (ql < nq) {
-                    if constexpr (sizeof(C) == 16) cp_async16(b + ql * LD + kz, SP + q0 + ql + Q * kz);
-                    else cp_async8(reinterpret_cast<double*>(b + ql * LD + kz), reinterpret_cast<const double*>(SP + q0 + ql + Q * kz));
-                }
-            }
-        }
-        cp_async_commit();  // an empty group past the end keeps the group count uniform
-    };
-    const T sc = SIGN < 0 ? (T)(1.0 / (double)N) : (T)1.0;
-    issue(blockIdx.x, buf0);
-    int cur = 0;
-#pragma unroll 1
-    for (long long tile = blockIdx.x; tile < ntile; tile += gridDim.x, cur ^= 1) {
-        C* const bc = buf0 + cur * (TQ * LD);
-        issue(tile + gridDim.x, buf0 + (cur ^ 1) * (TQ * LD));
-        cp_async_wait_group<1>();  // this tile's copies (all but the newest group) have landed
-        const long long q0 = tile * TQ;
-        const int nq = (int)min((long long)TQ, Q - q0);
-        block_fft4s<N1, N2, SIGN>(bc, nq, LD, twz_of<C>(g));  // starts and ends with a block barrier
-#pragma unroll 1
-        for (int p = threadIdx.x; p < TQ * N; p += NT) {
-            const int kz = p / TQ, ql = p - kz * TQ;
-            if (ql < nq) {
-                C v = bc[ql * LD + kz];
-                if (SIGN < 0) { v.x = v.x * sc; v.y = v.y * sc; }
-                SP[q0 + ql + Q * kz] = v;
-            }
-        }
-        __syncthreads();  // the buffer is the copy target of the iteration after next
-    }
-    cp_async_wait_group<0>();
 }
 
 // ---------------------------------------------------------------------------
@@ -935,60 +889,52 @@ __global__ void __launch_bounds__(YS_NT) k_ysolve_2w(Geo g, C* SP, double2* G, c
 }
 
 // ---------------------------------------------------------------------------
+// Inverse x transform of PX_TJ y rows, two rows a, b packed as one complex line Z = A + iB.  Thread
+// (pair, j1) forms its first-pass values Z_k, k = j1 + N1 j2, from the stored half spectra in registers
+// (Z_{L-k} = conj A_k + i conj B_k; imaginary parts of the k = 0 and k = L/2 coefficients are dropped, as
+// FFT99 does for ISIGN = +1): a coefficient is read for k and for L - k, the second time from L1.  Per
+// step 0.108 -> 0.068 ms at 256 x 192 x 128, 0.60 -> 0.55 at 384 x 256 x 384 (FP32: 0.35 -> 0.26).  The
+// forward transform keeps its staged form: it reads five field rows per line, more than the registers
+// beside a first-pass transform can hold in flight (0.173 -> 0.300 ms at 192 x 128 x 192).
 template <int N1, int N2, typename C>
-__global__ void __launch_bounds__(PX_NT, px_minb<C>()) k_fftx_inv(Geo g, const C* __restrict__ SP,
-                                                    typename CReal<C>::T* __restrict__ DPH) {
+__global__ void __launch_bounds__(px_nt<N1>(), (px_rminb<C, N1>())) k_fftx_inv(Geo g, const C* __restrict__ SP,
+                                                                         typename CReal<C>::T* __restrict__ DPH) {
     pdl_wait();
     using T = typename CReal<C>::T;
     extern __shared__ __align__(16) unsigned char smp_raw[];
     C* smc = reinterpret_cast<C*>(smp_raw);
-    const int L = g.L, M = g.M, LH = g.LH;
-    const int LD = fft4s_ld(L);
-    const int j0 = 1 + blockIdx.x * PX_TJ;
-    const int k = blockIdx.y;
-    const int nj = min(PX_TJ, M - j0 + 1);
-    const int np = (nj + 1) >> 1;
-    // The block's spectrum rows are requested into L2 first, 128-byte lines spread over the
-    // threads, so that the loads of the item loop below (a few in flight per thread) find them
-    // there: 0.657 -> 0.610 ms per 384 x 256 x 384 FP64 step.  (The same for the five field rows
-    // of k_div_fftx made it slower, 1.40 -> 1.47 ms.)
+    constexpr int L = N1 * N2, LH = L / 2 + 1, LD = L + N2 + 1;
+    const int M = g.M, j0 = 1 + blockIdx.x * PX_TJ, k = blockIdx.y;
     {
-        const int lpr = (LH * (int)sizeof(C) + 127) / 128;
-        for (int t = threadIdx.x; t < nj * lpr; t += PX_NT) {
-            const int r = t / lpr, c = t - r * lpr;
-            prefetch_l2(reinterpret_cast<const char*>(SP + (long long)LH * ((j0 + r - 1) + (long long)M * k)) + 128 * c);
-        }
-    }
-    // Z_k = A_k + i B_k with A_{L-k} = conj A_k; imaginary parts of the k = 0 and
-    // k = L/2 coefficients are dropped, as FFT99 does for ISIGN = +1.  Each
-    // stored coefficient is read once and gives Z at k and at L - k.
-#pragma unroll 2
-    for (int p = threadIdx.x; p < np * LH; p += PX_NT) {
-        const int pair = p / LH, ks = p - pair * LH;
-        const int ja = j0 + 2 * pair;
-        const bool hasb = 2 * pair + 1 < nj;
-        C a = SP[ks + (long long)LH * ((ja - 1) + (long long)M * k)];
-        C b = hasb ? SP[ks + (long long)LH * ((ja) + (long long)M * k)] : mkc((T)0, (T)0);
-        C* line = smc + pair * LD;
-        if (ks == 0 || 2 * ks == L) {
-            a.y = (T)0;
-            b.y = (T)0;
-        } else {
-            line[L - ks] = mkc(a.x - (-b.y), (-a.y) + b.x);
-        }
-        line[ks] = mkc(a.x - b.y, a.y + b.x);
-    }
-    block_fft4s<N1, N2, +1>(smc, np, LD, twx_of<C>(g));
-    // DPH rows with 16-byte stores (W consecutive points per thread; L is a multiple of 4)
-    constexpr int W = V16<T>::W;
-    const int LV = L / W;
-    for (int p = threadIdx.x; p < nj * LV; p += PX_NT) {
-        const int jl = p / LV, i0 = (p - jl * LV) * W;
-        const C* z = smc + (jl >> 1) * LD + i0;
-        T v[W];
+        const int j1 = threadIdx.x % N1, pair = threadIdx.x / N1;
+        const C* ra = SP + (long long)LH * ((j0 + 2 * pair - 1) + (long long)M * k);
+        const C* rb = ra + LH;
+        C v[N2];
 #pragma unroll
-        for (int e = 0; e < W; ++e) v[e] = (jl & 1) ? z[e].y : z[e].x;
-        st16(DPH + pidx(g, i0, j0 + jl, k), v);
+        for (int j2 = 0; j2 < N2; ++j2) {
+            const int q = j1 + N1 * j2;
+            const bool up = q > L / 2;
+            const int ks = up ? L - q : q;
+            C a = ra[ks], b = rb[ks];
+            if (ks == 0 || 2 * ks == L) {
+                a.y = (T)0;
+                b.y = (T)0;
+            }
+            v[j2] = up ? mkc(a.x - (-b.y), (-a.y) + b.x) : mkc(a.x - b.y, a.y + b.x);
+        }
+        fft_first<N1, N2, +1>(v, smc + pair * LD, j1, twx_of<C>(g));
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < PX_TJ / 2 * N2; t += px_nt<N1>()) {
+        const int pair = t / N2, k2 = t - pair * N2;
+        C v[N1];
+        fft_second<N1, +1>(v, smc + pair * LD, k2);
+        T* da = DPH + pidx(g, k2, j0 + 2 * pair, k);
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) {
+            da[N2 * k1] = v[k1].x;
+            da[N2 * k1 + L] = v[k1].y;  // the next row (x-periodic layout: row stride L)
+        }
     }
 }
 

@@ -512,29 +512,24 @@ int chapsim_dump_write(chapsim_ctx_t* ctx, const char* path_prefix, int32_t iter
  *          whatever is forced;
  *   bit 8: tile shape of the z sweep (periodic channel only), 0 = 32
  *          consecutive x lines per tile, 1 = 16;
- *   bit 9: with the chained transforms, the z transforms as persistent
- *          blocks that load their next tile while transforming the current
- *          one (periodic channel only; timed as a third pressure-stage form);
+ *   bits 9 and 12: kept as forced, no effect (they chose among forms of the
+ *          chained z transform; there is one);
  *   bit 10: z-sweep tile layout (periodic channel only), 0 = each x line
  *          contiguous in shared memory, 1 = lines interleaved in pairs (one
  *          copy instruction per two points); in FP64, whose sweeps hold
  *          their lines in registers, bits 10 and 11 are kept but have no
  *          effect;
- *   bit 11: the same for the y sweep (Q is restored after its trials);
- *   bit 12: with the chained transforms, each z-transform block also
- *          requests into L2 the tile of the block one wave later (timed as a
- *          fourth pressure-stage form).
+ *   bit 11: the same for the y sweep (Q is restored after its trials).
  * choice receives the kept setting in the same bit form; ms[19] (may be NULL)
  * the mean durations of y-solve (hybrid, sequential), right-hand sides
  * (fused, split, bulk-staged), pressure stage up to DPH (chained, fused;
  * 1e30 where a variant does not apply), the two-way y-solve, the
  * sequential y-solve at one block per SM (1e30 where it does not apply) and
  * the scan y-solve, the z sweep with 32- and with 16-line tiles (0 where it
- * does not apply), the pressure stage with the double-buffered z
- * transforms, the wide right-hand side (1e30 where it does not apply), and
+ * does not apply), the chained pressure stage again, the wide right-hand side (1e30 where it does not apply), and
  * the z sweep with pair-interleaved 32- and 16-line tiles, the y sweep with
- * line-contiguous and pair-interleaved tiles, and the pressure stage with
- * the z transforms' wave-ahead requests.
+ * line-contiguous and pair-interleaved tiles, and the chained pressure stage
+ * once more.
  * CONVH0 is restored after the trial launches.  Without the call a mixed-
  * precision context runs with all bits 0, an FP64 one with bits 6 and 8, and
  * bit 3 where a plane fits one block. */
