@@ -122,12 +122,14 @@ __device__ void factor_dispatch(int S, const C& cf, int lane, T* fac) {
     }
 }
 
-// Table of the FP64 z sweep (k_zsweep_reg).  The cyclic system with rows (a, 1 - 2a, a), a <= 0, factors
-// into c (1 - rho E^-1)(1 - rho E) with c = (1 + 2|a| + sqrt(1 + 4|a|)) / 2 and rho = |a| / c < 1 (E the
-// shift by one row), i.e. two first-order recurrences.  f[0] = 1/c, f[1] = 1/(1 - rho^n), f[2 + k] =
-// rho^k for k = 0..sr (sr rows per segment).
+// Table of an FP64 cyclic sweep (k_zsweep_reg, warp_cyc_apply).  The system with rows (a, 1 - 2a, a), a <= 0,
+// factors into c (1 - rho E^-1)(1 - rho E) with c = (1 + 2|a| + sqrt(1 + 4|a|)) / 2 and rho = |a| / c < 1 (E
+// the shift by one row), i.e. two first-order recurrences.  f[0] = 1/c, f[1] = 1/(1 - rho^n), f[2 + k] =
+// rho^k for k = 0..sr (sr rows per segment), then q^(2^s), q = rho^sr, s = 0..4.
 #define ZT_POW 2
-__device__ __forceinline__ void zsweep_table(double a, int n, int sr, int lane, double* __restrict__ f) {
+#define ZT_Q(sr) (ZT_POW + (sr) + 1)
+#define ZT_N(sr) (ZT_Q(sr) + 5)
+__device__ __forceinline__ void cyc_table(double a, int n, int sr, int lane, double* __restrict__ f) {
     const double m = -a;
     const double c = (1.0 + 2.0 * m + sqrt(1.0 + 4.0 * m)) * 0.5;
     const double rho = m / c;
@@ -137,6 +139,13 @@ __device__ __forceinline__ void zsweep_table(double a, int n, int sr, int lane, 
         if (k < lane) p *= rho;
     }
     if (lane <= sr) f[ZT_POW + lane] = p;
+    if (lane == sr) {
+        double q = p;
+        for (int s = 0; s < 5; ++s) {
+            f[ZT_Q(sr) + s] = q;
+            q *= q;
+        }
+    }
     if (lane == 0) {
         f[0] = 1.0 / c;
         f[1] = 1.0 / (1.0 - pn);
@@ -194,8 +203,12 @@ template <typename T>
 __device__ __forceinline__ void factor_set(const Geo& g, double dt, int ns, int set, T* f, int lane) {
     const double facoe = 0.5 * g.talp[ns] * dt * g.cvisc * 1.0 / 1.0;
     if constexpr (sizeof(T) == 8) {
+        if (set == FSET_X) {
+            cyc_table(-facoe * g.dxqi, g.L, g.L / 32, lane, f);  // MOMFA1_X_tg :72-78
+            return;
+        }
         if (set == FSET_Z) {
-            zsweep_table(1.0 * (-facoe * g.dzqi), g.N, seg_rows(g.N), lane, f);  // MOMFA2_Z_tg :133-155
+            cyc_table(1.0 * (-facoe * g.dzqi), g.N, seg_rows(g.N), lane, f);  // MOMFA2_Z_tg :133-155
             return;
         }
         if (set >= FSET_Y) {  // MOMFA3_Y_tg :172-238
@@ -231,6 +244,88 @@ __device__ __forceinline__ void factor_set(const Geo& g, double dt, int ns, int 
         YCoef cf{g.amvr + comp * (g.M + 2), g.acvr + comp * (g.M + 2), g.apvr + comp * (g.M + 2), facoe};
         factor_dispatch<false>(g.M / 32, cf, lane, f);
     }
+}
+
+// FP64 cyclic x lines of one warp, lane l owning rows l S .. l S + S - 1: the two recurrences of cyc_table
+// along each lane's rows, the lanes' carries combined by a cyclic shuffle scan (5 steps in powers of
+// rho^S, closed by 1/(1 - rho^n)).  NR lines at once.  S + 8 factors, the same for all lanes, where the
+// Thomas/PCR hybrid (warp_tdma_apply_n) reads 5 S + 20 per lane: right-hand side + x sweep 71 -> 67 us per
+// launch at 128^3, 0.97 -> 0.95 ms at 384 x 256 x 384.
+template <int S, int NR>
+__device__ __forceinline__ void warp_cyc_apply(double (&d)[NR][S], const double* __restrict__ tab, int lane) {
+    const double ic = tab[0], ring = tab[1], rho = tab[ZT_POW + 1];
+    const double* pw = tab + ZT_POW;
+    const double* pq = tab + ZT_Q(S);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) d[r][0] *= ic;
+#pragma unroll
+    for (int k = 1; k < S; ++k)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) d[r][k] = fma(rho, d[r][k - 1], d[r][k] * ic);
+    double c[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) c[r] = __shfl_sync(0xffffffffu, d[r][S - 1], (lane - 1) & 31);
+#pragma unroll
+    for (int s = 0; s < 5; ++s)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) c[r] = fma(pq[s], __shfl_sync(0xffffffffu, c[r], (lane - (1 << s)) & 31), c[r]);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) c[r] *= ring;
+#pragma unroll
+    for (int k = 0; k < S; ++k)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) d[r][k] = fma(pw[k + 1], c[r], d[r][k]);
+#pragma unroll
+    for (int k = S - 2; k >= 0; --k)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) d[r][k] = fma(rho, d[r][k + 1], d[r][k]);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) c[r] = __shfl_sync(0xffffffffu, d[r][0], (lane + 1) & 31);
+#pragma unroll
+    for (int s = 0; s < 5; ++s)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) c[r] = fma(pq[s], __shfl_sync(0xffffffffu, c[r], (lane + (1 << s)) & 31), c[r]);
+#pragma unroll
+    for (int r = 0; r < NR; ++r) c[r] *= ring;
+#pragma unroll
+    for (int k = 0; k < S; ++k)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) d[r][k] = fma(pw[S - k], c[r], d[r][k]);
+}
+
+// The x sweep of one (j, k): its three lines in segment-padded shared memory at base, base + ls, base + 2 ls;
+// line 1 (v) is solved but written back only when keep1 (MOMFA1_X_tg starts at N2I = 2 for v).
+template <int S>
+__device__ __forceinline__ void x_solve3(double* base, int ls, bool keep1, const double* __restrict__ tab, int lane) {
+    double d[3][S];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int k = 0; k < S; ++k) d[c][k] = base[c * ls + lane * (S + 1) + k];
+    warp_cyc_apply<S, 3>(d, tab, lane);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        if (c == 1 && !keep1) continue;
+#pragma unroll
+        for (int k = 0; k < S; ++k) base[c * ls + lane * (S + 1) + k] = d[c][k];
+    }
+}
+template <int S>
+__device__ __forceinline__ void x_solve3(float* base, int ls, bool keep1, const float* __restrict__ fac, int lane) {
+    warp_tdma_apply_smem3<S, true>(base, ls, keep1, fac, lane);
+}
+template <int S>
+__device__ __forceinline__ void x_solve1(double* base, const double* __restrict__ tab, int lane) {
+    double d[1][S];
+#pragma unroll
+    for (int k = 0; k < S; ++k) d[0][k] = base[lane * (S + 1) + k];
+    warp_cyc_apply<S, 1>(d, tab, lane);
+#pragma unroll
+    for (int k = 0; k < S; ++k) base[lane * (S + 1) + k] = d[0][k];
+}
+template <int S>
+__device__ __forceinline__ void x_solve1(float* base, const float* __restrict__ fac, int lane) {
+    warp_tdma_apply_smem<S, true>(base, fac, lane);
 }
 
 // Factor tables of one substep (block b computes set b: 0 x sweep, 1 z
@@ -495,7 +590,7 @@ __global__ void __launch_bounds__(RHS_WPB * 32, RHS_MINB_P(R, PV)) k_rhs_xsweep(
     __syncwarp();
     // cyclic x sweeps of this warp's three lines (MOMFA1_X_tg starts at N2I = 2 for v)
     const R* fx = fac + FSET_X * FAC_SET;
-    warp_tdma_apply_smem3<S, true>(sl, LS, j >= 2, fx, lane);  // the three components together
+    x_solve3<S>(sl, LS, j >= 2, fx, lane);  // the three components together
     __syncwarp();
 #pragma unroll
     for (int kk = 0; kk < S; ++kk) {
@@ -523,6 +618,7 @@ __global__ void __launch_bounds__(RHS_WPB * 32, RHS_MINB_P(R, PV)) k_rhs_xsweep(
     if (is_last) {
         __threadfence();
         double s = 0.0;
+#pragma unroll 16  // loads in flight: up to 192 partials per thread, added in order
         for (int t = threadIdx.x; t < (int)gridDim.x; t += RHS_WPB * 32) s += __ldcg(partial + t);
         s = block_sum<RHS_WPB * 32>(s, sred);
         if (threadIdx.x == 0) {
@@ -647,7 +743,7 @@ __global__ void __launch_bounds__(SWEEP_NT, (zsweep_blocks<R, S>())) k_zsweep(Ge
 // ---------------------------------------------------------------------------
 // FP64 cyclic z sweep in registers.  A block solves TI consecutive x lines of one (component, j): thread
 // (il, seg) owns the SR consecutive z rows of segment seg of line il, so every global access is a
-// row piece of TI doubles and nothing is staged or transposed.  The two recurrences of zsweep_table
+// row piece of TI doubles and nothing is staged or transposed.  The two recurrences of cyc_table
 // run along the segment in registers; the segments' carries go through NSEG x TI doubles of shared
 // memory, where each thread sums the preceding (following) segments' totals around the ring by Horner's
 // rule in rho^SR and closes the ring with 1/(1 - rho^n).
@@ -1046,7 +1142,7 @@ __global__ void __launch_bounds__(XS_NT) k_xsweep(Geo g, R* __restrict__ RHS, co
 #pragma unroll
     for (int q = 0; q < S; ++q) sl[seg_pos<S>(lane + 32 * q)] = v[q];
     __syncwarp();
-    warp_tdma_apply_smem<S, true>(sl, fac + FSET_X * FAC_SET, lane);
+    x_solve1<S>(sl, fac + FSET_X * FAC_SET, lane);
     __syncwarp();
 #pragma unroll
     for (int q = 0; q < S; ++q) base[lane + 32 * q] = sl[seg_pos<S>(lane + 32 * q)];

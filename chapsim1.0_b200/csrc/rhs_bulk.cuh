@@ -42,12 +42,14 @@ template <typename R>
 __host__ __device__ inline size_t rb_warp_bytes(int L) {
     return (size_t)rb_warp_elems(L) * sizeof(R);
 }
-// After the warps' regions, the block keeps the x sweep's factor table: its
-// 5S+20 values per lane are read in every line's solve, and with the stages
-// filling the shared memory the L1 is too small to hold them (they came from
-// L2, inside the sweep's dependency chain).
+// After the warps' regions, the block keeps the x sweep's factor table (S + 8
+// numbers in FP64, 5S+20 values per lane in FP32): it is read in every line's
+// solve, and with the stages filling the shared memory the L1 is too small to
+// hold it (it came from L2, inside the sweep's dependency chain).
 template <typename R>
-__host__ __device__ inline size_t rb_fac_bytes(int L) { return (size_t)TF_NF(L / 32) * 32 * sizeof(R); }
+__host__ __device__ constexpr int rb_fac_elems(int L) { return sizeof(R) == 8 ? ZT_N(L / 32) : TF_NF(L / 32) * 32; }
+template <typename R>
+__host__ __device__ inline size_t rb_fac_bytes(int L) { return (size_t)rb_fac_elems<R>(L) * sizeof(R); }
 // warps per block that fit beside the factor table, given the block's
 // shared-memory limit less the kernel's static shared memory
 template <typename R>
@@ -138,7 +140,7 @@ __global__ void __launch_bounds__(rb_wmax<R>() * 32, 1) k_rhs_xsweep_bulk(Geo g,
     R* const sfx = reinterpret_cast<R*>(rb_raw) + (size_t)nw * rb_warp_elems(L);
     {
         const R* fx = fac + FSET_X * FAC_SET;
-        for (int t = threadIdx.x; t < TF_NF(S) * 32; t += blockDim.x) sfx[t] = fx[t];
+        for (int t = threadIdx.x; t < rb_fac_elems<R>(L); t += blockDim.x) sfx[t] = fx[t];
     }
     __syncthreads();
     double bulk = 0.0;
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(rb_wmax<R>() * 32, 1) k_rhs_xsweep_bulk(Geo g,
             gn = rb_geo(g, 1 + (line + stride) % M);  // arrives during this line's x sweep
         }
         // cyclic x sweeps of this line's three components (MOMFA1_X_tg starts at N2I = 2 for v)
-        warp_tdma_apply_smem3<S, true>(sl, LS, j >= 2, sfx, lane);  // the three components together
+        x_solve3<S>(sl, LS, j >= 2, sfx, lane);  // the three components together
         __syncwarp();
         R* Rl = RHS + iidx(g, 0, j, k);
 #pragma unroll
@@ -231,9 +233,13 @@ __global__ void __launch_bounds__(rb_wmax<R>() * 32, 1) k_rhs_xsweep_bulk(Geo g,
     __syncthreads();
     if (is_last) {
         __threadfence();
+        // the partials' loads together (the stages are free by now), their sum in index order
+        double* const sp = reinterpret_cast<double*>(rb_raw);
+        for (int t = threadIdx.x; t < (int)gridDim.x; t += blockDim.x) sp[t] = __ldcg(partial + t);
+        __syncthreads();
         if (threadIdx.x == 0) {
             double s = 0.0;
-            for (int t = 0; t < (int)gridDim.x; ++t) s += __ldcg(partial + t);
+            for (int t = 0; t < (int)gridDim.x; ++t) s += sp[t];
             st->bulksum = s;
             st->ctr = 0u;
         }
