@@ -447,10 +447,24 @@ size_t smem_ysc(const Geo& g) {
     return (size_t)(2 * YW_L * (g.M + 33)) * sizeof(C) + (size_t)2 * (g.M + 32) * sizeof(double);
 }
 
+// the scan variant's factors, in the order of the kernel that reads them
+void ysolve_scan_factors(chapsim_ctx* ctx) {
+    const Geo& g = ctx->g;
+    const int nb = (int)(((long long)g.LH * g.N + 127) / 128);
+    if (ctx->prec == CHAPSIM_PREC_MIXED) k_ysolve_scan_factors<<<nb, 128, 0, ctx->stream>>>(g, ctx->YF3);
+    else k_ysolve_reg_factors<<<nb, 128, 0, ctx->stream>>>(g, ctx->YF3);
+}
+
 template <typename C>
 void launch_ysolve_scan(chapsim_ctx* ctx) {
     const Geo& g = ctx->g;
     const long long nl = (long long)g.LH * g.N;
+    if (ctx->prec != CHAPSIM_PREC_MIXED) {
+        DISPATCH_SEG(g.M, (launch_pdl(ctx->pdl, k_ysolve_reg<NSEG * SR / yseg_rows(NSEG * SR), yseg_rows(NSEG * SR)>, (int)(nl / YR_TI),
+                                      YR_TI * (NSEG * SR / yseg_rows(NSEG * SR)), 0, ctx->stream, g, ctx->SP,
+                                      (const double*)ctx->YF3)));
+        return;
+    }
     const int nb = (int)std::min<long long>((nl + YW_L - 1) / YW_L, ctx->nsm);  // persistent: one block per SM
     DISPATCH_S(g.M / 32, (launch_pdl(ctx->pdl, k_ysolve_scan<S, C>, nb, YW_NT, smem_ysc<C>(g), ctx->stream, g,
                                      spec<C>(ctx), (const double*)ctx->YF3)));
@@ -1209,12 +1223,12 @@ int chapsim_gpu_init(const chapsim_grid_t* grid, const chapsim_coefs_t* cf, cons
     k_ysolve_zero_factors<<<1, 32, 0, ctx->stream>>>(g, ctx->yz);
     INIT_CK(cudaGetLastError());
     if (ctx->prec == CHAPSIM_PREC_FP64 && !xio) {
-        // FP64 contexts start with the y-solve by affine scans: faster than the hybrid at every size measured
-        // (warp hybrid / scans: 12.7 / 6.3 us at 64^3, 43.0 / 21.1 at 128^3, 79.4 / 32.0 at 192 x 256 x 96,
-        // 449 / 264 at 384 x 256 x 384).  Mixed-precision contexts start with the hybrid: their FP32 fields
+        // FP64 contexts start with the y-solve by affine scans: faster than the others at every size measured
+        // (warp hybrid / scans in registers: 43 / 14 us at 128^3, 74 / 22 at 192 x 128 x 192, 449 / 133 at
+        // 384 x 256 x 384).  Mixed-precision contexts start with the hybrid: their FP32 fields
         // are reproduced to the bit.
         INIT_CK(cudaMalloc(&ctx->YF3, (size_t)g.LH * M * N * sizeof(double)));
-        k_ysolve_scan_factors<<<(int)(((long long)g.LH * N + 127) / 128), 128, 0, ctx->stream>>>(g, ctx->YF3);
+        ysolve_scan_factors(ctx);
         INIT_CK(cudaGetLastError());
         ctx->ysolve_kind = 4;
     }
@@ -2762,7 +2776,7 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
     }
     if (!ctx->YF3) {
         CK(cudaMalloc(&ctx->YF3, nsp * sizeof(double)));
-        k_ysolve_scan_factors<<<4 * ctx->nsm, 128, 0, s>>>(g, ctx->YF3);
+        ysolve_scan_factors(ctx);
         CK(cudaGetLastError());
     }
     // the variants are timed on the spectral array the time step uses (FP32 in the mixed-precision step)

@@ -889,6 +889,113 @@ __global__ void __launch_bounds__(YS_NT) k_ysolve_2w(Geo g, C* SP, double2* G, c
 }
 
 // ---------------------------------------------------------------------------
+// The FP64 form of the scan variant: the same two recurrences over the sequential factors, held in
+// registers by the layout of the FP64 y sweep (k_ysweep_reg, momentum.cuh): thread (il, seg) owns SR
+// consecutive y rows of mode line il, YR_TI lines (consecutive kx) per block, so the spectrum and the pivots
+// are read and written as row pieces, with nothing staged or transposed; the segments' carries and
+// multipliers change over through shared memory and are summed by Horner's rule.  Pivots in the
+// spectrum's own order, F[kx + LH (t + M kz)] = PP_t; the multipliers A_t PP_t and H_t = C_t PP_t are formed
+// from them.  Bound by the bytes of the spectrum and the pivots: scan kernel / this, us per launch, 39 / 22 at
+// 192 x 128 x 192, 43 / 27 at 256 x 192 x 128, 264 / 133 at 384 x 256 x 384 (sequential form 213; floor of its 40
+// bytes per mode row 117), 23 / 14 at 128^3.
+constexpr int YR_TI = 8;
+__global__ void k_ysolve_reg_factors(Geo g, double* __restrict__ F) {
+    const int M = g.M, LH = g.LH;
+    const long long nl = (long long)LH * g.N;
+    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nl; q += (long long)gridDim.x * blockDim.x) {
+        const int kz = (int)(q / LH), kx = (int)(q - (long long)kz * LH);
+        const double shift = (-g.ak1[kx] / 1.0 - g.ak3[kz]);
+        double* f = F + kx + (long long)LH * M * kz;
+        double hp = 0.0;
+        for (int j = 1; j <= M; ++j) {
+            const double pp = 1.0 / ((g.acph[j] + shift) - (j > 1 ? hp * g.amph[j] : 0.0));
+            hp = (j == M || (j == 1 && q == 0)) ? 0.0 : g.apph[j] * pp;
+            f[(long long)LH * (j - 1)] = pp;
+        }
+    }
+}
+
+template <int NSEG, int SR>
+__global__ void __launch_bounds__(YR_TI * NSEG, (SR > 12 ? 512 : SR > 8 ? 640 : 768) / (YR_TI * NSEG)) k_ysolve_reg(Geo g, double2* __restrict__ SP,
+                                                                                                   const double* __restrict__ F) {
+    pdl_wait();
+    constexpr int M = NSEG * SR, TI = YR_TI;
+    __shared__ double2 sc[NSEG][TI];            // the segments' last (first) values
+    __shared__ double sm[NSEG][TI], sam[M], sap[M];  // and their products of multipliers; AMPH, APPH
+    const int LH = g.LH;
+    const int il = threadIdx.x % TI, seg = threadIdx.x / TI;
+    const unsigned q = blockIdx.x * TI + il;    // mode line; LH N is a multiple of 32
+    const unsigned kz = q / (unsigned)LH, kx = q - kz * (unsigned)LH;
+    const long long o = kx + (long long)LH * (seg * SR + (long long)M * kz);
+    double2* s = SP + o;
+    const double* f = F + o;
+    double2 d[SR];
+    double pp[SR];
+#pragma unroll
+    for (int r = 0; r < SR; ++r) d[r] = s[(long long)LH * r];
+#pragma unroll
+    for (int r = 0; r < SR; ++r) pp[r] = f[(long long)LH * r];
+    for (int t = threadIdx.x; t < M; t += TI * NSEG) {
+        sam[t] = t == 0 ? 0.0 : -g.amph[t + 1];
+        sap[t] = t == M - 1 ? 0.0 : -g.apph[t + 1];
+    }
+    __syncthreads();
+    const double* am = sam + seg * SR;
+    const double* ap = sap + seg * SR;
+    // the zero mode (kx = kz = 0): phi_hat(y_1) = 0, and row 1 does not couple
+    const bool zero = q == 0 && seg == 0;
+    if (zero) d[0] = make_double2(0.0, 0.0);
+    d[0] = c_scale(d[0], pp[0]);
+    double w = am[0] * pp[0];
+#pragma unroll
+    for (int r = 1; r < SR; ++r) {
+        const double a = am[r] * pp[r];
+        d[r] = make_double2(fma(a, d[r - 1].x, d[r].x * pp[r]), fma(a, d[r - 1].y, d[r].y * pp[r]));
+        w *= a;
+    }
+    sc[seg][il] = d[SR - 1];
+    sm[seg][il] = w;
+    __syncthreads();
+    double2 c = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int m = 0; m < NSEG - 1; ++m)
+        if (m < seg) {
+            const double2 v = sc[m][il];
+            const double x = sm[m][il];
+            c = make_double2(fma(c.x, x, v.x), fma(c.y, x, v.y));
+        }
+#pragma unroll
+    for (int r = 0; r < SR; ++r) {
+        c = c_scale(c, am[r] * pp[r]);
+        d[r] = make_double2(d[r].x + c.x, d[r].y + c.y);
+    }
+    w = ap[SR - 1] * pp[SR - 1];
+#pragma unroll
+    for (int r = SR - 2; r >= 0; --r) {
+        const double h = (zero && r == 0) ? 0.0 : ap[r] * pp[r];
+        d[r] = make_double2(fma(h, d[r + 1].x, d[r].x), fma(h, d[r + 1].y, d[r].y));
+        w *= h;
+    }
+    __syncthreads();  // the forward carries have been read
+    sc[seg][il] = d[0];
+    sm[seg][il] = w;
+    __syncthreads();
+    c = make_double2(0.0, 0.0);
+#pragma unroll 4
+    for (int m = NSEG - 1; m >= 1; --m)
+        if (m > seg) {
+            const double2 v = sc[m][il];
+            const double x = sm[m][il];
+            c = make_double2(fma(c.x, x, v.x), fma(c.y, x, v.y));
+        }
+#pragma unroll
+    for (int r = SR - 1; r >= 0; --r) {
+        c = c_scale(c, (zero && r == 0) ? 0.0 : ap[r] * pp[r]);
+        s[(long long)LH * r] = make_double2(d[r].x + c.x, d[r].y + c.y);
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Inverse x transform of PX_TJ y rows, two rows a, b packed as one complex line Z = A + iB.  Thread
 // (pair, j1) forms its first-pass values Z_k, k = j1 + N1 j2, from the stored half spectra in registers
 // (Z_{L-k} = conj A_k + i conj B_k; imaginary parts of the k = 0 and k = L/2 coefficients are dropped, as

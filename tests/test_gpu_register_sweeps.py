@@ -1,6 +1,7 @@
-"""The line sweeps in registers at every line length, against the oracle's
-sequential line solves: the FP64 z and y sweeps of the periodic channel (both
-tile widths) and the Crank-Nicolson sweeps of the main domain.
+"""The line solves in registers at every line length, against the oracle's
+sequential ones: the FP64 z and y sweeps of the periodic channel (both tile
+widths), the Crank-Nicolson sweeps of the main domain, and the FP64 Poisson
+y-solve with the register transforms.
 
 REN = 2 makes the implicit operators stiff (|a| = F / dz^2 from 1 to 190 at
 these grids, where the recurrences' ratio rho approaches 1 and carries travel
@@ -77,3 +78,22 @@ def test_stiff_main_domain_sweeps_match_oracle(shape):
     for q in range(3):
         e = float(np.abs(Gg[q] - Go[q]).max() / np.abs(Go[q]).max())
         assert e <= 1e-11, (q, e)
+
+
+@pytest.mark.parametrize("shape", [(64, 32, 32), (32, 64, 96), (384, 96, 64), (96, 128, 384), (128, 192, 128),
+                                   (256, 256, 192), (192, 384, 256)])
+def test_poisson_solve_matches_oracle(shape):
+    """The default FP64 solve (inverse x and both z transforms on registers, the y-solve by affine maps in
+    registers) at every line length, 1e-12 of the oracle as for the other y-solves."""
+    L, M, N = shape
+    s = channel_setup(L, M, N, 2 * math.pi, math.pi, 2.0, 2800.0)
+    o = Oracle(L, M, N, 2 * math.pi, math.pi, 2.0, 2800.0, threads=8)
+    rhs = np.random.default_rng(19).standard_normal((N, M, L))
+    full = np.zeros((N, M + 2, L))
+    full[:, 1:M + 1, :] = rhs
+    ref = o.poisson(full)
+    o.close()
+    c = gpu.ChannelTG(s)
+    got = c.FFT99_POIS3D_periodicxz(rhs)
+    c.close()
+    assert float(np.abs(got[:, 1:M + 1] - ref[:, 1:M + 1]).max() / np.abs(ref[:, 1:M + 1]).max()) <= 1e-12
