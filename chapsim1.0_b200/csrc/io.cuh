@@ -667,26 +667,51 @@ __global__ void __launch_bounds__(PX_NT, PX_MINB) k_io_div_fftx(Geo g, const F* 
     // wdiv: 0.25 + pres_epslon with iWeightedPre = 1, else 1 (an exact division)
     const double coe0 = 1.0 / st->dt / g.talp[ns] / wdiv;
     const double coe1 = g.dxi / 1.0;
-#pragma unroll 4
-    for (int p = threadIdx.x; p < 2 * np * L; p += PX_NT) {
-        const int jl = p / L, i = p - jl * L;
-        const int pair = jl >> 1, part = jl & 1;
-        double val = 0.0;
-        if (jl < nj) {
-            const int j = j0 + jl;
-            const long long c = pidx(g, i, j, k);
-            const double u = G[c], up = G[pidx(g, wrapp(i, L), j, k)];
-            const double v = G[c + g.FS], vp = G[c + g.FS + L];
-            const double w = G[c + 2 * g.FS], wp = G[pidx(g, i, j, kp) + 2 * g.FS];
-            const double coe2 = g.dyfi[j] / 1.0;
-            const double DIVX = (up - u) * coe1, DIVY = (vp - v) * coe2, DIVZ = (wp - w) * g.dzi;
-            const double DTRHO = DRHO ? DRHO[c] / 1.0 : 0.0;
-            const double DQ = DIVX + DIVY + DIVZ + DTRHO;
-            val = DQ * coe0;
-            RHSLL[iidx(g, i, j, k)] = val;
+    // one item = two consecutive points of both rows of a packed pair, by vector loads (rows start at multiples
+    // of L, which is a multiple of 32; M is one too, so every row of the tile exists): twice the bytes in
+    // flight of single loads, 0.32 -> 0.24 ms per step at 256 x 192 x 128 (FP32 storage 0.31 -> 0.21)
+    auto ld2 = [](const F* p, double (&o)[2]) {
+        if constexpr (sizeof(F) == 8) {
+            const double2 v = *reinterpret_cast<const double2*>(p);
+            o[0] = v.x; o[1] = v.y;
+        } else {
+            const float2 v = *reinterpret_cast<const float2*>(p);
+            o[0] = v.x; o[1] = v.y;
         }
-        double2* line = smc + pair * LD;
-        if (part == 0) line[i].x = val; else line[i].y = val;
+    };
+    const int LV = L / 2;
+#pragma unroll 2
+    for (int p = threadIdx.x; p < np * LV; p += PX_NT) {
+        const int pair = p / LV, i0 = (p - pair * LV) * 2;
+        double val[2][2];
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+            const int j = j0 + 2 * pair + part;
+            const long long c = pidx(g, i0, j, k);
+            double u[2], v[2], vp[2], w[2], wp[2], dr[2] = {0.0, 0.0};
+            ld2(G + c, u);
+            ld2(G + c + g.FS, v);
+            ld2(G + c + g.FS + L, vp);
+            ld2(G + c + 2 * g.FS, w);
+            ld2(G + pidx(g, i0, j, kp) + 2 * g.FS, wp);
+            const double un = G[pidx(g, i0 + 2 == L ? 0 : i0 + 2, j, k)];
+            if (DRHO) {
+                const double2 d = *reinterpret_cast<const double2*>(DRHO + c);
+                dr[0] = d.x / 1.0; dr[1] = d.y / 1.0;
+            }
+            const double coe2 = g.dyfi[j] / 1.0;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const double up = e == 0 ? u[1] : un;
+                const double DIVX = (up - u[e]) * coe1, DIVY = (vp[e] - v[e]) * coe2, DIVZ = (wp[e] - w[e]) * g.dzi;
+                const double DQ = DIVX + DIVY + DIVZ + dr[e];
+                val[part][e] = DQ * coe0;
+            }
+            *reinterpret_cast<double2*>(RHSLL + iidx(g, i0, j, k)) = make_double2(val[part][0], val[part][1]);
+        }
+        double2* line = smc + pair * LD + i0;
+        line[0] = make_double2(val[0][0], val[1][0]);
+        line[1] = make_double2(val[0][1], val[1][1]);
     }
     block_fft4s<N1, N2, -1>(smc, np, LD, g.twx);
     const double sc = 0.5 / (double)L;
