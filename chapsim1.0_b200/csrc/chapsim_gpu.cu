@@ -896,8 +896,9 @@ void launch_io_rhs(chapsim_ctx* ctx, const IoFieldsT<float>& f, int ns) {
     k_io_rhs<CN, float><<<ctx->io_grid, IO_NT, 0, ctx->stream>>>(ctx->g, f, ctx->part_rhs, ctx->st, ns);
 }
 
+// more: another substep of the same step follows at once
 template <typename F>
-void launch_io_substep_t(chapsim_ctx* ctx, int ns) {
+void launch_io_substep_t(chapsim_ctx* ctx, int ns, bool more) {
     const Geo& g = ctx->g;
     cudaStream_t s = ctx->stream;
     if (ctx->thermal) launch_thermal_substep_t<F>(ctx, ns);
@@ -941,13 +942,16 @@ void launch_io_substep_t(chapsim_ctx* ctx, int ns) {
     prof_mark(ctx);
     DISPATCH_FFT(g.L, (k_fftx_inv<FN1, FN2, double2><<<grp, px_nt<FN1>(), smem_px(g), s>>>(g, ctx->SP, ctx->DPH)));
     prof_mark(ctx);
-    k_io_correct<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->DPH, ctx->st, ns, ctx->ivis ? ctx->RHSLL : nullptr);
+    if (more && ctx->thermal)
+        k_io_correct<false, F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->DPH, ctx->st, ns, ctx->ivis ? ctx->RHSLL : nullptr);
+    else
+        k_io_correct<true, F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->DPH, ctx->st, ns, ctx->ivis ? ctx->RHSLL : nullptr);
     prof_mark(ctx);
     ctx->launches += 8;
 }
-void launch_io_substep(chapsim_ctx* ctx, int ns) {
-    if (io_mixed(ctx)) launch_io_substep_t<float>(ctx, ns);
-    else launch_io_substep_t<double>(ctx, ns);
+void launch_io_substep(chapsim_ctx* ctx, int ns, bool more = false) {
+    if (io_mixed(ctx)) launch_io_substep_t<float>(ctx, ns, more);
+    else launch_io_substep_t<double>(ctx, ns, more);
 }
 
 // ------------------------- inflow/outflow main domain ------------------------
@@ -1012,7 +1016,7 @@ void launch_xio_substep(chapsim_ctx* ctx, int ns, cudaEvent_t tg_read = nullptr)
         k_xio_dctx_inv<<<nrb, XIO_NT, smem_xd(g), s>>>(g, ctx->SP, ctx->xio_cf + (size_t)g.LI * g.LI, ctx->DPH);
     }
     prof_mark(ctx);
-    k_io_correct<double><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->DPH, ctx->st, ns, nullptr);
+    k_io_correct<true, double><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->DPH, ctx->st, ns, nullptr);
     prof_mark(ctx);
     ctx->launches += 12;
 }
@@ -1070,7 +1074,7 @@ int build_step_graph(chapsim_ctx* ctx) {
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     if (ctx->domain == 2) {
         launch_io_step_start(ctx);
-        for (int ns = 1; ns <= 3; ++ns) launch_io_substep(ctx, ns);
+        for (int ns = 1; ns <= 3; ++ns) launch_io_substep(ctx, ns, ns < 3);
     } else {
         launch_step_start(ctx);
         for (int ns = 1; ns <= 3; ++ns) launch_substep(ctx, ns, false);
@@ -1861,7 +1865,7 @@ int chapsim_profile_steps(chapsim_ctx_t* ctx, int32_t nsteps, double dt0, double
         ctx->prof_n = 0;
         if (ctx->domain == 2) {
             launch_io_step_start(ctx);
-            for (int ns = 1; ns <= 3; ++ns) launch_io_substep(ctx, ns);
+            for (int ns = 1; ns <= 3; ++ns) launch_io_substep(ctx, ns, ns < 3);
         } else {
             launch_step_start(ctx);
             for (int ns = 1; ns <= 3; ++ns) launch_substep(ctx, ns, false);
