@@ -200,11 +200,12 @@ __device__ __forceinline__ double eng_divg(const Geo& g, const F* G, int i, int 
 // Of G0 only its divergence is ever used, and it is the div(G) of the previous call (G does not change between
 // DENSITY_TIME_DERIVATION and G0_io = G_io): DIVG0 holds that, one word per point read and written where
 // the three-component copy took three of each.  17 words per point instead of the 27 of three
-// kernels; 1.10 -> 0.59 ms per step at 256 x 192 x 128 (FP64).
+// kernels; 1.10 -> 0.59 ms per step at 256 x 192 x 128 (FP64), and 0.53 with four blocks per SM (64
+// registers instead of 78; FP32 storage 0.54 -> 0.42).
 // mpart (inflow/outflow domain, else NULL): per-block sums of DrhoDtP / DYFI for the interior mass
 // rate of CHK_MassConsv_io (src/processing/CHK_conservation.f90:41-53)
 template <typename F>
-__global__ void __launch_bounds__(IO_NT) k_eng_state(Geo g, IoFieldsT<F> f, ThermoFields t, int ns, double* __restrict__ mpart) {
+__global__ void __launch_bounds__(IO_NT, 4) k_eng_state(Geo g, IoFieldsT<F> f, ThermoFields t, int ns, double* __restrict__ mpart) {
     __shared__ double sred[32];
     const long long tot = io_points(g);
     double ms = 0.0;
