@@ -74,7 +74,7 @@ __global__ void __launch_bounds__((p2_nt<SpecT<R>, NX1 * NX2 * NZ1 * NZ2>()), 1)
         const double w = W[c], wp = W[pidx(g, i, j, wrapp(k, N))];
         const double dv = (up - u) * coe1 + (vp - v) * coe2 + (wp - w) * g.dzi;
         const double val = dv * coe0;
-        RHSLL[iidx(g, i, j, k)] = (R)val;
+        if constexpr (sizeof(R) == 4) RHSLL[iidx(g, i, j, k)] = (R)val;  // FP64: see k_correct
         C* line = smc + (k >> 1) * LDX;
         if ((k & 1) == 0) line[i].x = (T)val; else line[i].y = (T)val;
     }
