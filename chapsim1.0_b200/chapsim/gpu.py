@@ -316,7 +316,7 @@ class ChannelTG:
         # variant bits in use (chapsim_autotune): what the library starts with
         self.choice = 0
         if precision == "fp64" and self.IDOMAIN == 1:
-            self.choice = 64 | 256 | (8 if plane_in_one_block(setup.L, setup.N, precision) else 0)
+            self.choice = 64 | 256 | (6 if setup.L >= 192 else 4 if setup.L >= 64 else 0)
         if precision not in PRECISIONS:
             raise ValueError(f"precision must be one of {sorted(PRECISIONS)}")
         self.precision = precision

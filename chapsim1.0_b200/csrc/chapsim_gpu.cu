@@ -540,10 +540,11 @@ int configure_kernels(chapsim_ctx* ctx) {
     ctx->zs_tw = ctx->prec != CHAPSIM_PREC_MIXED ? 16 : 32;
     int rc = ctx->prec == CHAPSIM_PREC_MIXED ? configure_momentum<float>(ctx) : configure_momentum<double>(ctx);
     if (rc) return rc;
-    // and the fused plane transforms in FP64 where a plane fits one block (chained / fused pressure stage:
-    // 21.6 / 19.6 us at 64^3, 84.2 / 71.0 at 128^3, 162 / 143 at 192 x 256 x 96); the cluster form is slower
-    // than the chained transforms (303 / 426 at 256 x 128 x 256)
-    if (ctx->domain == 1 && ctx->prec != CHAPSIM_PREC_MIXED && plane_fft_ok<double2>(g)) ctx->plane_kind = 1;
+    // FP64 right-hand sides before any tuning: one fused form per range of L (ms per step, fused / bulk-staged /
+    // wide): L = 32 fused (0.074 / 0.078 at 32^3), 64 to 128 bulk-staged (0.133 / 0.132 at 64^3, 0.637 / 0.559 / 0.605
+    // at 128^3, 1.140 / 1.002 at 96 x 192 x 192), from 192 on the wide one (1.382 / 1.362 / 1.296 at 192 x 128 x 192,
+    // 2.71 / 3.06 / 2.53 at 384 x 128 x 192)
+    if (ctx->domain == 1 && ctx->prec != CHAPSIM_PREC_MIXED) ctx->k1_kind = g.L >= 192 ? 3 : g.L >= 64 && ctx->rb_nw > 0 ? 2 : 0;
     // the FP64 spectral stage serves the standalone Poisson solve and the main domain in every precision
     DISPATCH_FFT(g.L, CK(set_smem(k_fftx_inv<FN1, FN2, double2>, smem_px(g))));
     DISPATCH_FFT(g.L, CK(set_smem(k_fftx_from_rhs<FN1, FN2>, smem_px(g))));
@@ -3008,7 +3009,9 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
             ctx->fz_pipe = (force & 512) != 0;
             ctx->fz_prefetch = (force & 4096) != 0;
         } else {
-            ctx->plane_kind = tp[1] < tp[0] ? 1 : 0;
+            // the trials launch from the host, whose pace flatters the form with fewer kernels on small grids (64^3:
+            // 15.7 chained, 16.0 fused here, 0.132 against 0.138 ms per captured step)
+            ctx->plane_kind = tp[1] < 0.9f * tp[0] ? 1 : 0;
             ctx->fz_pipe = ctx->fz_prefetch = false;
         }
         tp[2] = tp[3] = tp[0];

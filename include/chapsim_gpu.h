@@ -531,8 +531,8 @@ int chapsim_dump_write(chapsim_ctx_t* ctx, const char* path_prefix, int32_t iter
  * line-contiguous and pair-interleaved tiles, and the chained pressure stage
  * once more.
  * CONVH0 is restored after the trial launches.  Without the call a mixed-
- * precision context runs with all bits 0, an FP64 one with bits 6 and 8, and
- * bit 3 where a plane fits one block. */
+ * precision context runs with all bits 0, an FP64 one with bits 6 and 8 and
+ * with right-hand side 0 (L = 32), 2 (64 to 128) or 3 (longer lines). */
 int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choice, float* ms);
 
 /* An ensemble of independent periodic channels (any grids and precisions, one
