@@ -156,7 +156,7 @@ struct chapsim_ctx {
     double* yz = nullptr;         // zero-mode factors of the warp y-solve (Geo::yz)
     double* YF = nullptr;         // factors of the sequential y-solve, 2 M doubles per line (when chosen)
     double* YF2 = nullptr;        // factors of the two-way y-solve, 2 M doubles per line (when chosen)
-    double* YF3 = nullptr;        // pivots of the scan y-solve, M doubles per line, line by line (when chosen)
+    double* YF3 = nullptr;        // pivots of the scan y-solve, in the spectrum's order (when chosen)
     int ysolve_kind = 0;          // 0: warp Thomas/PCR hybrid, 1: sequential Thomas, 2: two-way, 3: sequential with
                                   // the forward intermediate in shared memory at one block per SM, 4: warp affine
                                   // scans over the sequential factors (chapsim_autotune)
@@ -442,11 +442,6 @@ void launch_ysolve_2w(chapsim_ctx* ctx) {
                spec<C>(ctx), ctx->SP, ctx->YF2);
 }
 
-template <typename C>
-size_t smem_ysc(const Geo& g) {
-    return (size_t)(2 * YW_L * (g.M + 33)) * sizeof(C) + (size_t)2 * (g.M + 32) * sizeof(double);
-}
-
 // the scan variant's factors, in the order of the kernel that reads them
 void ysolve_scan_factors(chapsim_ctx* ctx) {
     const Geo& g = ctx->g;
@@ -459,15 +454,15 @@ template <typename C>
 void launch_ysolve_scan(chapsim_ctx* ctx) {
     const Geo& g = ctx->g;
     const long long nl = (long long)g.LH * g.N;
+    // (a mixed-precision context solves its FP64 spectra, the main domain's and the Poisson entry's, by scans as well)
     if (ctx->prec != CHAPSIM_PREC_MIXED) {
         DISPATCH_SEG(g.M, (launch_pdl(ctx->pdl, k_ysolve_reg<NSEG * SR / yseg_rows(NSEG * SR), yseg_rows(NSEG * SR)>, (int)(nl / YR_TI),
                                       YR_TI * (NSEG * SR / yseg_rows(NSEG * SR)), 0, ctx->stream, g, ctx->SP,
                                       (const double*)ctx->YF3)));
-        return;
+    } else {
+        DISPATCH_S(g.M / 32, (launch_pdl(ctx->pdl, k_ysolve_scan<S, C>, (int)(nl / YC_L), 32 * YC_L, 0, ctx->stream, g,
+                                         spec<C>(ctx), (const double*)ctx->YF3)));
     }
-    const int nb = (int)std::min<long long>((nl + YW_L - 1) / YW_L, ctx->nsm);  // persistent: one block per SM
-    DISPATCH_S(g.M / 32, (launch_pdl(ctx->pdl, k_ysolve_scan<S, C>, nb, YW_NT, smem_ysc<C>(g), ctx->stream, g,
-                                     spec<C>(ctx), (const double*)ctx->YF3)));
 }
 
 template <typename C>
@@ -518,7 +513,6 @@ int configure_momentum(chapsim_ctx* ctx) {
     DISPATCH_FFT(g.L, CK(set_smem(k_div_fftx<R, FN1, FN2>, smem_px<C>(g))));
     DISPATCH_FFT(g.L, CK(set_smem(k_fftx_inv<FN1, FN2, C>, smem_px<C>(g))));
     DISPATCH_S(g.M / 32, CK(set_smem(k_ysolve_warp<S, C>, smem_yw<C>(g))));
-    DISPATCH_S(g.M / 32, CK(set_smem(k_ysolve_scan<S, C>, smem_ysc<C>(g))));
     CK(set_smem(k_ysolve_seq<C, false>, smem_ysolve_seq(g.M, false)));
     CK(set_smem(k_ysolve_seq<C, true>, smem_ysolve_seq(g.M, ysolve_seq_kg(g) || ysolve_seq_kg1(g))));
     CK(set_smem(k_ysolve_2w<C>, smem_ysolve_seq()));
@@ -551,7 +545,6 @@ int configure_kernels(chapsim_ctx* ctx) {
     DISPATCH_FFT(g.L, CK(set_smem(k_io_div_fftx<FN1, FN2, double>, smem_px(g))));
     DISPATCH_FFT(g.L, CK(set_smem(k_io_div_fftx<FN1, FN2, float>, smem_px(g))));
     DISPATCH_S(g.M / 32, CK(set_smem(k_ysolve_warp<S, double2>, smem_yw<double2>(g))));
-    DISPATCH_S(g.M / 32, CK(set_smem(k_ysolve_scan<S, double2>, smem_ysc<double2>(g))));
     CK(set_smem(k_ysolve_seq<double2, false>, smem_ysolve_seq(g.M, false)));
     CK(set_smem(k_ysolve_seq<double2, true>, smem_ysolve_seq(g.M, ysolve_seq_kg(g) || ysolve_seq_kg1(g))));
     CK(set_smem(k_ysolve_2w<double2>, smem_ysolve_seq()));

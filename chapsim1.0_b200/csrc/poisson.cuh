@@ -367,24 +367,24 @@ __global__ void __launch_bounds__(YW_NT, 1) k_ysolve_warp(Geo g, C* __restrict__
 }
 
 // ---------------------------------------------------------------------------
-// Fifth y-solve variant: the sequential recurrence's factors (the same pivots
-// PP and multipliers H as k_ysolve_seq_factors; k_ysolve_scan_factors stores
-// the pivots line by line, F[q*M + t] = PP_t, and the kernel forms each
-// H_t = APPH(t+1) PP_t, H_0 = C_0 / PP_0, H_{M-1} = 0, with the factor
-// kernel's own operations, so only half the factor bytes are read) turn both sweeps
-// into first-order linear recurrences,
-//   forward   g_t = (r_t - A_t g_{t-1}) PP_t      (g_0 = r_0 / PP_0, r_0 = 0 on the zero mode)
+// Fifth y-solve variant, in mixed-precision contexts (FP64 ones have k_ysolve_reg): the sequential recurrence's
+// factors (the pivots PP and multipliers H of k_ysolve_seq_factors; k_ysolve_scan_factors stores the pivots in
+// the spectrum's order, F[kx + LH (t + M kz)] = PP_t, F = B_0 at t = 0, and the kernel forms each
+// H_t = APPH(t+1) PP_t, H_0 = C_0 / B_0, H_{M-1} = 0, with the factor kernel's own operations) turn both
+// sweeps into first-order linear recurrences,
+//   forward   g_t = (r_t - A_t g_{t-1}) PP_t      (g_0 = r_0 / B_0, r_0 = 0 on the zero mode)
 //   backward  x_t = g_t - H_t x_{t+1}             (H_{M-1} = 0),
-// which one warp per line evaluates as affine scans: lane l owns rows
-// lS .. lS+S-1, composes its rows' maps, the 32 lane maps are combined by a
-// shuffle scan (5 steps), and each lane then runs its rows' recurrence
-// sequentially from its incoming value, in the reference's operation order.
-// Only the spectrum is read and written (plus the factors): the forward
-// intermediate stays in registers, where the sequential variant moves it
-// through memory.  Lines are staged as in k_ysolve_warp (persistent,
-// double-buffered groups of YW_L lines, one warp per line).  The lane maps are
-// combined in tree order, so the result agrees with the sequential recurrence
-// to rounding (1e-12 of the oracle on the Poisson problem).
+// evaluated as affine scans over 32 segments of S rows per line: a segment composes its rows' maps, the 32
+// maps of a line are combined by a shuffle scan (5 steps), and each segment then runs its rows' recurrence
+// sequentially from its incoming value, in the reference's operation order.  Thread (il, seg) holds
+// segment seg of mode line il in registers, YC_L lines (consecutive kx) per block, so the spectrum and the
+// pivots move as row pieces and nothing is staged; the maps change over to one lane per segment
+// through shared memory.  The maps are combined in tree order, so the result agrees with the
+// sequential recurrence to rounding (1e-12 of the oracle on the Poisson problem).  Bound by latency: at
+// 384x256x384 the FP32 spectrum, read and written, and the pivots are 24 B a mode, 0.07 ms of memory a solve;
+// 8 lines a block (four row pieces of 64 B per warp) take 0.125 ms, the warp per line with its lines staged
+// in shared memory that this replaces 0.162 (128^3: 15.6 against 18.9 us).
+constexpr int YC_L = 8;
 
 __global__ void k_ysolve_scan_factors(Geo g, double* __restrict__ F) {
     const int M = g.M, LH = g.LH;
@@ -395,169 +395,133 @@ __global__ void k_ysolve_scan_factors(Geo g, double* __restrict__ F) {
         const double b = g.acph[1] + shift;
         const double c = q == 0 ? 0.0 : g.apph[1];
         double hp = c / b;
-        double* f = F + q * M;
+        double* f = F + kx + (long long)LH * M * kz;
         f[0] = b;
         for (int j = 2; j <= M; ++j) {
             const double pp = 1.0 / ((g.acph[j] + shift) - hp * g.amph[j]);
             hp = j < M ? g.apph[j] * pp : 0.0;
-            f[j - 1] = pp;
+            f[(long long)LH * (j - 1)] = pp;
         }
     }
 }
 
 template <int S, typename C>
-__global__ void __launch_bounds__(YW_NT, 1) k_ysolve_scan(Geo g, C* __restrict__ SP, const double* __restrict__ F) {
+__global__ void __launch_bounds__(32 * YC_L, 2) k_ysolve_scan(Geo g, C* __restrict__ SP, const double* __restrict__ F) {
     pdl_wait();
-    extern __shared__ __align__(16) unsigned char ysc_raw[];
-    static_assert(YW_NT == 32 * YW_L, "one warp per line of a group");
-    const int M = 32 * S, LH = g.LH;
-    const int LS = M + 33;
-    C* const stage[2] = {reinterpret_cast<C*>(ysc_raw), reinterpret_cast<C*>(ysc_raw) + YW_L * LS};
-    // AMPH(t+1) at t + t / S: a lane reads rows lS .. lS+S-1, and the pad after every S rows
-    // puts the lanes' rows on different banks (lane-strided reads of the unpadded rows made
-    // 36 M bank conflicts per launch at 384 x 256 x 384)
-    double* const sam = reinterpret_cast<double*>(reinterpret_cast<C*>(ysc_raw) + 2 * YW_L * LS);
-    double* const sap = sam + (M + 32);  // APPH(t+1), the same layout
-    for (int t = threadIdx.x; t < M; t += YW_NT) {
+    constexpr int M = 32 * S, TI = YC_L, LD = 33;
+    __shared__ double sA[TI * LD], sBx[TI * LD], sBy[TI * LD];
+    __shared__ double sam[M + 32], sap[M + 32];  // AMPH(t+1), APPH(t+1) at t + t / S: the segments' rows on different banks
+    const int LH = g.LH;
+    const int il = threadIdx.x % TI, seg = threadIdx.x / TI;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned q = blockIdx.x * TI + il;  // LH N is a multiple of 32
+    const unsigned kz = q / (unsigned)LH, kx = q - kz * (unsigned)LH;
+    const int r0 = seg * S, s0 = seg * (S + 1);  // the segment's first row and its operator-row slot
+    const long long o = kx + (long long)LH * (r0 + (long long)M * kz);
+    C* s = SP + o;
+    const double* f = F + o;
+    double2 d[S];
+    double pp[S], hh[S];
+#pragma unroll
+    for (int k = 0; k < S; ++k) d[k] = to_d2(s[(long long)LH * k]);
+#pragma unroll
+    for (int k = 0; k < S; ++k) pp[k] = __ldg(f + (long long)LH * k);
+    for (int t = threadIdx.x; t < M; t += 32 * TI) {
         sam[t + t / S] = g.amph[t + 1];
         sap[t + t / S] = g.apph[t + 1];
     }
-    const long long nl = (long long)LH * g.N;
-    const long long ngr = (nl + YW_L - 1) / YW_L;
-    const int ls = threadIdx.x % YW_L, js = threadIdx.x / YW_L;
-    constexpr int RS = YW_NT / YW_L;
-    auto line_ptr = [&](long long q) {
-        const int kz = (int)(q / LH), kx = (int)(q - (long long)kz * LH);
-        return SP + kx + (long long)LH * ((long long)M * kz);
-    };
-    auto issue = [&](long long gr, C* st) {
-        if (gr < ngr) {
-            const long long q = gr * YW_L + ls;
-            if (q < nl) {
-                const C* src = line_ptr(q);
-                for (int j = js; j < M; j += RS) cp_async_row(st + ls * LS + seg_pos<S>(j), src + (long long)LH * j);
-            }
-        }
-        cp_async_commit();
-    };
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = lane * S, s0 = lane * (S + 1);  // the lane's first row and its operator-row slot
-    issue(blockIdx.x, stage[0]);
-    int cur = 0;
-#pragma unroll 1
-    for (long long gr = blockIdx.x; gr < ngr; gr += gridDim.x, cur ^= 1) {
-        issue(gr + gridDim.x, stage[cur ^ 1]);
-        // this warp's line pivots (coalesced: the warp reads 32 S contiguous doubles)
-        const long long q = gr * YW_L + warp;
-        double pp[S], hh[S];
-        if (q < nl) {
-            const double* f = F + q * M + r0;
-            if constexpr (S % 2 == 0) {
+    __syncthreads();
 #pragma unroll
-                for (int k = 0; k < S; k += 2) {
-                    const double2 a = __ldg(reinterpret_cast<const double2*>(f + k));
-                    pp[k] = a.x; pp[k + 1] = a.y;
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < S; ++k) pp[k] = __ldg(f + k);
-            }
-        }
-        cp_async_wait_group<1>();
-        __syncthreads();  // (also the first iteration's barrier for sam and sap)
-        if (q < nl) {
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-                const int t = r0 + k;
-                if (t == 0) hh[k] = (q == 0 ? 0.0 : sap[0]) / pp[0];
-                else hh[k] = t < M - 1 ? sap[s0 + k] * pp[k] : 0.0;
-            }
-        }
-        C* const st = stage[cur];
-        if (q < nl) {
-            C* base = st + warp * LS + lane * (S + 1);
-            double2 d[S];
-#pragma unroll
-            for (int k = 0; k < S; ++k) d[k] = to_d2(base[k]);
-            if (q == 0 && lane == 0) d[0] = make_double2(0.0, 0.0);  // the zero mode's pinned first row
-            // forward: the lane's map g_out = A g_in + B over its rows (row 0 ignores g_in)
-            double A = 1.0;
-            double2 B = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-                const int t = r0 + k;
-                if (t == 0) {
-                    A = 0.0;
-                    B = make_double2(d[k].x / pp[k], d[k].y / pp[k]);
-                } else {
-                    const double al = -sam[s0 + k] * pp[k];
-                    B = make_double2(al * B.x + d[k].x * pp[k], al * B.y + d[k].y * pp[k]);
-                    A = al * A;
-                }
-            }
-            // inclusive scan over the lanes (lane 0's map first)
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const double Ap = __shfl_up_sync(0xffffffffu, A, o);
-                const double Bx = __shfl_up_sync(0xffffffffu, B.x, o), By = __shfl_up_sync(0xffffffffu, B.y, o);
-                if (lane >= o) {
-                    B = make_double2(A * Bx + B.x, A * By + B.y);
-                    A = A * Ap;
-                }
-            }
-            double2 gp = make_double2(__shfl_up_sync(0xffffffffu, B.x, 1), __shfl_up_sync(0xffffffffu, B.y, 1));
-            if (lane == 0) gp = make_double2(0.0, 0.0);
-            // the lane's rows from its incoming value, in the reference's order
-#pragma unroll
-            for (int k = 0; k < S; ++k) {
-                const int t = r0 + k;
-                if (t == 0) {
-                    gp = make_double2(d[k].x / pp[k], d[k].y / pp[k]);
-                } else {
-                    const double a = sam[s0 + k];
-                    gp = make_double2((d[k].x - a * gp.x) * pp[k], (d[k].y - a * gp.y) * pp[k]);
-                }
-                d[k] = gp;
-            }
-            // backward: x_t = g_t - H_t x_{t+1}; the lane's map gives its first row's x from the next lane's
-            // first row's (x_in): x = A x_in + B, composed from the lane's last row down
-            A = 1.0;
-            B = make_double2(0.0, 0.0);
-#pragma unroll
-            for (int k = S - 1; k >= 0; --k) {
-                const double ga = -hh[k];
-                B = make_double2(ga * B.x + d[k].x, ga * B.y + d[k].y);
-                A = ga * A;
-            }
-            // inclusive scan over the lanes from lane 31 down
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const double Ap = __shfl_down_sync(0xffffffffu, A, o);
-                const double Bx = __shfl_down_sync(0xffffffffu, B.x, o), By = __shfl_down_sync(0xffffffffu, B.y, o);
-                if (lane + o < 32) {
-                    B = make_double2(A * Bx + B.x, A * By + B.y);
-                    A = A * Ap;
-                }
-            }
-            double2 xn = make_double2(__shfl_down_sync(0xffffffffu, B.x, 1), __shfl_down_sync(0xffffffffu, B.y, 1));
-            if (lane == 31) xn = make_double2(0.0, 0.0);  // H_{M-1} = 0: the top row is its own g
-#pragma unroll
-            for (int k = S - 1; k >= 0; --k) {
-                xn = make_double2(d[k].x - hh[k] * xn.x, d[k].y - hh[k] * xn.y);
-                base[k] = from_d2<C>(xn);
-            }
-        }
-        __syncthreads();
-        {
-            const long long qs = gr * YW_L + ls;
-            if (qs < nl) {
-                C* dst = line_ptr(qs);
-                for (int j = js; j < M; j += RS) dst[(long long)LH * j] = st[ls * LS + seg_pos<S>(j)];
-            }
-        }
-        __syncthreads();
+    for (int k = 0; k < S; ++k) {
+        const int t = r0 + k;
+        if (t == 0) hh[k] = (q == 0 ? 0.0 : sap[0]) / pp[0];
+        else hh[k] = t < M - 1 ? sap[s0 + k] * pp[k] : 0.0;
     }
-    cp_async_wait_group<0>();
+    if (q == 0 && seg == 0) d[0] = make_double2(0.0, 0.0);  // the zero mode's pinned first row
+    // forward: the segment's map g_out = A g_in + B over its rows (row 0 ignores g_in)
+    double A = 1.0;
+    double2 B = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int k = 0; k < S; ++k) {
+        const int t = r0 + k;
+        if (t == 0) {
+            A = 0.0;
+            B = make_double2(d[k].x / pp[k], d[k].y / pp[k]);
+        } else {
+            const double al = -sam[s0 + k] * pp[k];
+            B = make_double2(al * B.x + d[k].x * pp[k], al * B.y + d[k].y * pp[k]);
+            A = al * A;
+        }
+    }
+    const int p = il * LD + seg, w = warp * LD + lane;  // this thread's segment; warp: line, lane: segment
+    sA[p] = A; sBx[p] = B.x; sBy[p] = B.y;
+    __syncthreads();
+    {   // inclusive scan over the segments (the first one's map first); each receives its predecessor's value
+        A = sA[w];
+        B = make_double2(sBx[w], sBy[w]);
+#pragma unroll
+        for (int n = 1; n < 32; n <<= 1) {
+            const double Ap = __shfl_up_sync(0xffffffffu, A, n);
+            const double Bx = __shfl_up_sync(0xffffffffu, B.x, n), By = __shfl_up_sync(0xffffffffu, B.y, n);
+            if (lane >= n) {
+                B = make_double2(A * Bx + B.x, A * By + B.y);
+                A = A * Ap;
+            }
+        }
+        double2 gp = make_double2(__shfl_up_sync(0xffffffffu, B.x, 1), __shfl_up_sync(0xffffffffu, B.y, 1));
+        if (lane == 0) gp = make_double2(0.0, 0.0);
+        sBx[w] = gp.x; sBy[w] = gp.y;
+    }
+    __syncthreads();
+    {   // the segment's rows from their incoming value, in the reference's order
+        double2 gp = make_double2(sBx[p], sBy[p]);
+#pragma unroll
+        for (int k = 0; k < S; ++k) {
+            const int t = r0 + k;
+            if (t == 0) {
+                gp = make_double2(d[k].x / pp[k], d[k].y / pp[k]);
+            } else {
+                const double a = sam[s0 + k];
+                gp = make_double2((d[k].x - a * gp.x) * pp[k], (d[k].y - a * gp.y) * pp[k]);
+            }
+            d[k] = gp;
+        }
+    }
+    // backward: x_t = g_t - H_t x_{t+1}; the segment's map gives its first row's x from the next segment's
+    // first row's (x_in): x = A x_in + B, composed from the segment's last row down
+    A = 1.0;
+    B = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int k = S - 1; k >= 0; --k) {
+        const double ga = -hh[k];
+        B = make_double2(ga * B.x + d[k].x, ga * B.y + d[k].y);
+        A = ga * A;
+    }
+    sA[p] = A; sBx[p] = B.x; sBy[p] = B.y;  // (this thread's own entries, read above)
+    __syncthreads();
+    {   // inclusive scan over the segments from the last one down
+        A = sA[w];
+        B = make_double2(sBx[w], sBy[w]);
+#pragma unroll
+        for (int n = 1; n < 32; n <<= 1) {
+            const double Ap = __shfl_down_sync(0xffffffffu, A, n);
+            const double Bx = __shfl_down_sync(0xffffffffu, B.x, n), By = __shfl_down_sync(0xffffffffu, B.y, n);
+            if (lane + n < 32) {
+                B = make_double2(A * Bx + B.x, A * By + B.y);
+                A = A * Ap;
+            }
+        }
+        double2 xn = make_double2(__shfl_down_sync(0xffffffffu, B.x, 1), __shfl_down_sync(0xffffffffu, B.y, 1));
+        if (lane == 31) xn = make_double2(0.0, 0.0);  // H_{M-1} = 0: the top row is its own g
+        sBx[w] = xn.x; sBy[w] = xn.y;
+    }
+    __syncthreads();
+    double2 xn = make_double2(sBx[p], sBy[p]);
+#pragma unroll
+    for (int k = S - 1; k >= 0; --k) {
+        xn = make_double2(d[k].x - hh[k] * xn.x, d[k].y - hh[k] * xn.y);
+        s[(long long)LH * k] = from_d2<C>(xn);
+    }
 }
 
 // ---------------------------------------------------------------------------

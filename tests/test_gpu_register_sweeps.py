@@ -1,7 +1,8 @@
 """The line solves in registers at every line length, against the oracle's
 sequential ones: the FP64 z and y sweeps of the periodic channel (both tile
-widths), the Crank-Nicolson sweeps of the main domain, and the FP64 Poisson
-y-solve with the register transforms.
+widths), the Crank-Nicolson sweeps of the main domain, the FP64 Poisson
+y-solve with the register transforms, and the scan y-solve of mixed-precision
+contexts.
 
 REN = 2 makes the implicit operators stiff (|a| = F / dz^2 from 1 to 190 at
 these grids, where the recurrences' ratio rho approaches 1 and carries travel
@@ -97,3 +98,21 @@ def test_poisson_solve_matches_oracle(shape):
     got = c.FFT99_POIS3D_periodicxz(rhs)
     c.close()
     assert float(np.abs(got[:, 1:M + 1] - ref[:, 1:M + 1]).max() / np.abs(ref[:, 1:M + 1]).max()) <= 1e-12
+
+
+@pytest.mark.parametrize("shape", [(64, 32, 32), (32, 64, 96), (384, 96, 64), (96, 128, 384), (128, 192, 128),
+                                   (256, 256, 192), (192, 384, 256)])
+def test_mixed_scan_matches_warp_solve(shape):
+    """The scan y-solve of a mixed-precision context against its warp solve at every line length, the FP64
+    spectrum of the Poisson entry included; held to the bound that an FP32 spectrum would meet, one ulp a
+    mode and log2(L N) 2^-24 < 1.1e-6 of the inverse transforms' rounding (2e-6)."""
+    L, M, N = shape
+    s = channel_setup(L, M, N, 2 * math.pi, math.pi, 2.0, 2800.0)
+    rhs = np.random.default_rng(23).standard_normal((N, M, L))
+    p = []
+    for force in (0, 64):
+        c = gpu.ChannelTG(s, precision="mixed")
+        assert c.autotune(force=force)[0] == force
+        p.append(c.FFT99_POIS3D_periodicxz(rhs)[:, 1:M + 1])
+        c.close()
+    assert float(np.abs(p[1] - p[0]).max() / np.abs(p[0]).max()) <= 2e-6
