@@ -827,7 +827,12 @@ void launch_thermal_substep_t(chapsim_ctx* ctx, int ns) {
     const Geo& g = ctx->g;
     cudaStream_t s = ctx->stream;
     IoFieldsT<F> f = io_fields_t<F>(ctx);
-    k_eng_rhs<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->tf, ctx->tp, ctx->st, ns);
+    if constexpr (sizeof(F) == sizeof(double)) {
+        const int chunk = eng_tile_chunk(g, ctx->nsm);
+        k_eng_rhs_tile<<<io_tile_blocks(g, chunk), IT_NT, 0, s>>>(g, f, ctx->tf, ctx->tp, ctx->st, ns, chunk);
+    } else {
+        k_eng_rhs<F><<<ctx->io_grid, IO_NT, 0, s>>>(g, f, ctx->tf, ctx->tp, ctx->st, ns);
+    }
     prof_mark(ctx);
     const size_t sm = prop_smem(ctx->tab.n);
     const long long tot = (long long)g.L * g.M * g.N, plane = 2LL * g.L * g.N;

@@ -2,7 +2,7 @@
 sequential ones: the FP64 z and y sweeps of the periodic channel (both tile
 widths), the Crank-Nicolson sweeps of the main domain, the FP64 Poisson
 y-solve with the register transforms, and the scan y-solve of mixed-precision
-contexts.
+contexts; and the energy equation's tiles.
 
 REN = 2 makes the implicit operators stiff (|a| = F / dz^2 from 1 to 190 at
 these grids, where the recurrences' ratio rho approaches 1 and carries travel
@@ -15,8 +15,9 @@ import math
 import numpy as np
 import pytest
 
+import oracle as orc
 from oracle import Oracle
-from chapsim import gpu
+from chapsim import gpu, thermo
 from chapsim.mesh import channel_setup
 from chapsim.fields import initial_field
 
@@ -116,3 +117,36 @@ def test_mixed_scan_matches_warp_solve(shape):
         p.append(c.FFT99_POIS3D_periodicxz(rhs)[:, 1:M + 1])
         c.close()
     assert float(np.abs(p[1] - p[0]).max() / np.abs(p[0]).max()) <= 2e-6
+
+
+@pytest.mark.parametrize("shape", [(32, 32, 32), (96, 64, 192), (128, 32, 384), (256, 96, 64), (384, 192, 32)])
+def test_energy_tiles_match_oracle(shape):
+    """Two heated steps over grids whose z chunks are short, long or uneven, constant flux at both walls; 1e-10 as
+    in the thermal step tests (which hold the isothermal walls)."""
+    L, M, N = shape
+    HX, HZ, REN = 2 * math.pi, math.pi, 2800.0
+    s = channel_setup(L, M, N, HX, HZ, 2.0, REN)
+    Q, PR = initial_field(s, 47, 0.1)
+    rows, T0 = thermo.synthetic_table()
+    tab = thermo.SplineTable.from_rows(rows, T0)
+    cthecd = 1.0 / REN / (tab.ref["M0"] * tab.ref["CP0"] / tab.ref["K0"])
+    DH = np.zeros((N, M + 2, L))
+    DH[:, 1:M + 1, :] = 1e-3 * np.random.default_rng(29).uniform(-1.0, 1.0, (N, M, L))
+    ones = np.ones((N, M + 2, L))
+    o = Oracle(L, M, N, HX, HZ, 2.0, REN, DT0=1e-3, DTMIN=1e-6, CFLGV=0.5, threads=8)
+    o.io_set_fields(Q, PR, ones, ones, ones)
+    ot = orc.PropTable(tab.lists)
+    o.thermal_enable(ot, DH, 0.5, 0.5, cthecd)
+    o.set_dt(1e-3)
+    assert o.io_run_steps(2)[0] == 0
+    to = o.thermal_get()
+    o.close()
+    c = gpu.ChannelIO(s)
+    c.upload_io(Q, PR, ones, ones, ones)
+    c.thermal_init(tab, DH, 0.5, 0.5, cthecd)
+    c.set_dt(1e-3)
+    c.advance(2, 1e-3, 1e-6, 0.5)
+    tg = c.download_thermal()
+    c.close()
+    for q in ("DH", "H", "T", "D", "M", "K", "CP"):
+        assert float(np.abs(tg[q] - to[q]).max() / np.abs(to[q]).max()) <= 1e-10, q
