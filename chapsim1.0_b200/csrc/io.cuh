@@ -6,12 +6,13 @@
 //
 //   k_io_props     DENSITY_Staggered + MU_Staggered (src/MASSFLUX_CALC_IO.f90:155-329), once per upload
 //   k_io_divu      DIVG_U_io (src/DIVG.f90:140-246): DivU = div(u)/3
-//   k_io_rhs<CN>   CONVECTION_X/Y/Z_io, VISCOUS_ALL_EXPLT_X/Y/Z_io (or VISCOUS_PAR_EXPLT_*), RHS_MOM_EXPLICIT_io
+//   k_io_rhs_tile<CN> (FP64), k_io_rhs<CN> (FP32 storage)
+//                  CONVECTION_X/Y/Z_io, VISCOUS_ALL_EXPLT_X/Y/Z_io (or VISCOUS_PAR_EXPLT_*), RHS_MOM_EXPLICIT_io
 //                  (RK combination, EXPLT0 update, pressure gradient, grid sum of the
-//                  bulk-forcing integrand), one thread per point and all components
+//                  bulk-forcing integrand), all components at once
 //   k_io_massflux  bulk forcing subtraction + MASSFLUX_CALC_io (G += RHS)
 //   k_io_div_fftx  DIVG_io (src/DIVG.f90:54-137) + forward x transform
-//   (shared)       k_fftz / k_ysolve_warp / k_fftz / k_fftx_inv of poisson.cuh: the
+//   (shared)       k_fftz / y-solve / k_fftz / k_fftx_inv of poisson.cuh: the
 //                  discrete problem of FISHPACK_POIS3D_SIMPLE (same AMPH/ACPH/APPH operator
 //                  and x/z eigenvalues); its singular kx = kz = 0 mode is fixed at
 //                  phi_hat(y_1) = 0, which shifts DPH and PR by a constant only

@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(XIO_NT) k_fill(double* __restrict__ p, long lo
 // the previous one reduces over the whole plane); partial results per block, reduced by every
 // block in block order (deterministic).  BC0: BC_CONV0(J, K, IDR) as [IDR][K][J]; state[0] =
 // U_OUTLET, state[1] = CHK_Mass_CONSV0_SCALING of this substep; part: 2 doubles per block.
-// The interior mass rate (sum of DrhoDtP / DYFI) comes from k_drhodt's block sums with the thermal
+// The interior mass rate (sum of DrhoDtP / DYFI) comes from k_eng_state's block sums with the thermal
 // solver on, and is zero without it.
 //   a: extremes of UCC = (u(L) + u(L+1)) / 2 (CONVCTION_OUTLET_U, method two)
 //   b: U_OUTLET = (max + min) / 2, the convective update of the outlet column (:36-58), and
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(XIO_NT) k_xio_outlet_b(Geo g, IoFields f, doub
     }
 }
 
-// mpart, nmp: the per-block sums of DrhoDtP / DYFI of k_drhodt (thermal solver on), else NULL
+// mpart, nmp: the per-block sums of DrhoDtP / DYFI of k_eng_state (thermal solver on), else NULL
 __global__ void __launch_bounds__(XIO_NT) k_xio_outlet_c(Geo g, IoFields f, const double* __restrict__ partb,
                                                          const double* __restrict__ mpart, int nmp,
                                                          double* __restrict__ state, DevState* __restrict__ st) {

@@ -4,15 +4,16 @@
 //
 // Kernel split (all three velocity components per kernel):
 //   k_factors    : per substep, the line-independent factor tables of the
-//                  x, z and y sweeps (warp_tdma_factor)
+//                  x, z and y sweeps (FP32: warp_tdma_factor; FP64: the
+//                  recurrences' ratios and multipliers)
 //   k_rhs_xsweep : convection (CONVECTION_X_tg :13-64, CONVECTION_Y_tg
 //                  :13-114, CONVECTION_Z_tg :13-103), RK combination,
 //                  viscous and pressure-gradient terms (RHS_CvLpGpS_tg
 //                  :97-161), CONVH0 update, the grid sum of the bulk-flux
 //                  forcing (:163-181), then the cyclic x sweep
 //                  (MOMFA1_X_tg, src/MOMFA_tg.f90:51-106); one warp per x line
-//   k_zsweep     : cyclic z sweep (MOMFA2_Z_tg :110-169)
-//   k_ysweep     : forcing subtraction, non-cyclic y sweep (MOMFA3_Y_tg
+//   k_zsweep_reg (FP64), k_zsweep (FP32): cyclic z sweep (MOMFA2_Z_tg :110-169)
+//   k_ysweep_reg (FP64), k_ysweep (FP32): forcing subtraction, non-cyclic y sweep (MOMFA3_Y_tg
 //                  :172-238) and Q += dQ (MOMFA_tg :38-44)
 // The reference subtracts the forcing DPGRNS before the x sweep.  The x and
 // z operators are circulant with rows summing to one, so a constant passes
@@ -1034,7 +1035,7 @@ __global__ void __launch_bounds__(RP_NT, sizeof(R) == 4 ? 3 : 2) k_rhs_point(Geo
     R* ring = reinterpret_cast<R*>(sm_raw);   // [slot][field][jj][ii]
     __shared__ double sred[32];
     __shared__ int is_last;
-    const int L = g.L, M = g.M, N = g.N;
+    const int N = g.N;
     const int ti = threadIdx.x % RT_I, tj = threadIdx.x / RT_I;
     const int i0 = blockIdx.x * RT_I, j0 = 1 + blockIdx.y * RT_J;
     const int k0 = blockIdx.z * kchunk, k1 = min(N, k0 + kchunk);

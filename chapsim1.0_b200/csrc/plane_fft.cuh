@@ -7,7 +7,7 @@
 // The chained form (k_div_fftx, k_fftz<-1>, ..., k_fftz<+1>, k_fftx_inv)
 // moves the spectrum through HBM between the x and the z transforms.  Here
 // one block owns a whole row j:
-//   k_div_fft2  DIVG_tg for the x-z plane of row j (RHSLLPHI written once),
+//   k_div_fft2  DIVG_tg for the x-z plane of row j (in FP32 RHSLLPHI too),
 //               x transform of z-line pairs (two real lines k = 2p, 2p+1
 //               packed into one complex line), unpacking into z lines of the
 //               half spectrum, z transform, spectrum of row j written once;
@@ -20,7 +20,7 @@
 // after the forward z transform) are those of the chained kernels; only the
 // pairing of real lines differs (z pairs here, y pairs there), which changes
 // round-off only.  The grid is one block per row (M blocks); the autotuner
-// keeps the chained form where that is faster.
+// keeps the chained form unless this one is more than a tenth faster.
 #pragma once
 #include "common.cuh"
 #include "fft.cuh"

@@ -6,12 +6,13 @@
 //   BC_WALL_PR_tg (src/BC_WALL.f90:293-361).
 //
 // Kernels:
-//   k_div_fftx   divergence of u* / (alpha dt) -> RHSLLPHI, then the real
+//   k_div_fftx   divergence of u* / (alpha dt) (-> RHSLLPHI in FP32), then the real
 //                x transform of every (j, k) line (two real lines packed in
 //                one complex FFT), times 1/L, into the spectral array
 //   k_fftz<S>    complex z transform of every (kx, j) line; forward pass
 //                multiplies by 1/N (UN3M)
-//   k_ysolve_warp per (kx, kz) tridiagonal solve in y with diagonal
+//   k_ysolve_warp, _seq, _2w, _scan, _reg
+//                per (kx, kz) tridiagonal solve in y with diagonal
 //                ACPH(j) - AK1(kx) - AK3(kz); zero mode pinned as in
 //                TDMA_PHI_COEF (:225-231) and :341-344, :387-389
 //                (phi_hat(0,y_1,0) = 0)

@@ -30,13 +30,6 @@ struct ConstCoef {
     __device__ __forceinline__ double B(int) const { return b; }
     __device__ __forceinline__ double C(int) const { return c; }
 };
-struct SmemCoef {  // per-row coefficients in shared memory
-    const double *a, *b, *c;
-    __device__ __forceinline__ double A(int r) const { return a[r]; }
-    __device__ __forceinline__ double B(int r) const { return b[r]; }
-    __device__ __forceinline__ double C(int r) const { return c[r]; }
-};
-
 struct Row4 { double al, be, ga, de; };
 
 __device__ __forceinline__ Row4 shfl_row(const Row4& r, int src) {
@@ -165,17 +158,6 @@ __device__ __forceinline__ void warp_tdma(double (&d)[S], const Coef& cf, int la
             for (int k = 1; k <= S - 2; ++k) d[k] = d[k] - ap[k] * y0 - cq[k] * u;
         }
     }
-}
-
-// Solve one line stored in shared memory at base[seg_pos<S>(r)], r = 0..32*S-1.
-template <int S, bool CYCLIC, class Coef>
-__device__ __forceinline__ void warp_tdma_smem(double* base, const Coef& cf, int lane) {
-    double d[S];
-#pragma unroll
-    for (int k = 0; k < S; ++k) d[k] = base[lane * (S + 1) + k];
-    warp_tdma<S, CYCLIC>(d, cf, lane);
-#pragma unroll
-    for (int k = 0; k < S; ++k) base[lane * (S + 1) + k] = d[k];
 }
 
 // ---------------------------------------------------------------------------
