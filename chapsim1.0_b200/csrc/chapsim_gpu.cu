@@ -199,6 +199,7 @@ struct chapsim_ctx {
     IoFieldsT<float> iof{};       // FP32 flow fields of the mixed-precision main-domain step (Q, PR, RHS: Qf, PRf, RHSf)
     int io_grid = 0;              // blocks of the IO point-wise kernels
     cudaGraphExec_t step_exec = nullptr;
+    unsigned graph_gen = 0;       // counts the calls of drop_step_graph (ensembles compare it)
     cudaEvent_t* prof_ev = nullptr;  // when set, an event is recorded after every kernel
     int prof_n = 0;
     int kernels_per_step = 0;
@@ -1062,6 +1063,18 @@ int check_device_error(chapsim_ctx* ctx) {
             return fail(ctx, CHAPSIM_ERR_TABLE_RANGE, "rho*h (or h) left the property table during the energy update");
         if (e & CHS_EBIT_MMA_TIMEOUT)
             return fail(ctx, CHAPSIM_ERR_TIMEOUT, "a bounded device wait (tensor-core commit or bulk copy) ran out of time");
+    }
+    return CHAPSIM_OK;
+}
+
+// The captured step graph holds the kernels' arguments, the pointers of their tables among them: a new
+// setting needs a new capture.  The counter tells the ensembles that the context is a member of.
+int drop_step_graph(chapsim_ctx* ctx) {
+    ++ctx->graph_gen;
+    if (ctx->step_exec) {
+        CK(cudaStreamSynchronize(ctx->stream));
+        cudaGraphExecDestroy(ctx->step_exec);
+        ctx->step_exec = nullptr;
     }
     return CHAPSIM_OK;
 }
@@ -1965,16 +1978,6 @@ int chapsim_rk_substep_io(chapsim_ctx_t* ctx, int32_t ns) {
     return CHAPSIM_OK;
 }
 
-// the captured step graph holds the kernels' arguments: a new setting needs a new capture
-static int drop_step_graph(chapsim_ctx* ctx) {
-    if (ctx->step_exec) {
-        CK(cudaStreamSynchronize(ctx->stream));
-        cudaGraphExecDestroy(ctx->step_exec);
-        ctx->step_exec = nullptr;
-    }
-    return CHAPSIM_OK;
-}
-
 int chapsim_set_buoyancy(chapsim_ctx_t* ctx, int32_t igravity, double f_a) {
     if (!ctx || ctx->domain < 2) return fail(ctx, CHAPSIM_ERR_BADARG, "context was not created for the main (IO) domain");
     if (igravity < -3 || igravity > 3 || !std::isfinite(f_a))
@@ -2455,11 +2458,7 @@ extern "C" int chapsim_thermal_init(chapsim_ctx_t* ctx, const double* dh, double
     if (io_mixed(ctx)) thermal_start<float>(ctx, fb);
     else thermal_start<double>(ctx, fb);
     CK(cudaGetLastError());
-    if (ctx->step_exec) {  // the captured step no longer matches
-        CK(cudaStreamSynchronize(s));
-        cudaGraphExecDestroy(ctx->step_exec);
-        ctx->step_exec = nullptr;
-    }
+    if (int rc = drop_step_graph(ctx)) return rc;
     return check_device_error(ctx);
 }
 
@@ -2722,12 +2721,7 @@ extern "C" int chapsim_thermal_use_mlp(chapsim_ctx_t* ctx, int32_t enable) {
         return fail(ctx, CHAPSIM_ERR_BADARG, "the inflow/outflow main domain updates its properties by table search");
     CK(cudaSetDevice(ctx->device));
     ctx->use_mlp = enable != 0;
-    if (ctx->step_exec) {
-        CK(cudaStreamSynchronize(ctx->stream));
-        cudaGraphExecDestroy(ctx->step_exec);
-        ctx->step_exec = nullptr;
-    }
-    return CHAPSIM_OK;
+    return drop_step_graph(ctx);
 }
 
 extern "C" int chapsim_mlp_judge(chapsim_ctx_t* ctx, double* max_rel_err) {
@@ -2766,6 +2760,7 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
     const Geo& g = ctx->g;
     cudaStream_t s = ctx->stream;
     CK(cudaStreamSynchronize(s));
+    if (int rc = drop_step_graph(ctx)) return rc;  // first: a table may be freed below, and a call after that fail
     const size_t nsp = (size_t)g.LH * g.M * g.N;
     if (!ctx->YF) {
         CK(cudaMalloc(&ctx->YF, 2 * nsp * sizeof(double)));
@@ -3014,10 +3009,6 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
         }
         tp[2] = tp[3] = tp[0];
     }
-    if (ctx->step_exec) {
-        cudaGraphExecDestroy(ctx->step_exec);
-        ctx->step_exec = nullptr;
-    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (choice)
@@ -3042,6 +3033,7 @@ struct chapsim_batch {
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> join;
     cudaGraphExec_t exec = nullptr;
+    std::vector<unsigned> gen;         // the members' graph_gen at the capture
     int kernels_per_step = 0;
     std::string err;
 };
@@ -3114,6 +3106,8 @@ int batch_capture(chapsim_batch_t* b) {
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return fail(ctx, CHAPSIM_ERR_CUDA, std::string("ensemble instantiate: ") + cudaGetErrorString(e));
     b->kernels_per_step = kernels;
+    b->gen.clear();
+    for (chapsim_ctx* c : b->ctx) b->gen.push_back(c->graph_gen);
     return CHAPSIM_OK;
 }
 }  // namespace
@@ -3125,6 +3119,12 @@ extern "C" int chapsim_batch_advance(chapsim_batch_t* b, int32_t nsteps, double 
         int rc = set_step_params(c, dt0, dtmin, cflgv);
         if (rc) return fail(nullptr, rc, c->err);
     }
+    // a member's setting that has changed since the capture (its tables may be freed) needs a new one
+    for (size_t i = 0; b->exec && i < b->ctx.size(); ++i)
+        if (b->ctx[i]->graph_gen != b->gen[i]) {
+            cudaGraphExecDestroy(b->exec);  // (every advance waits for the ensemble's stream)
+            b->exec = nullptr;
+        }
     if (!b->exec) {
         int rc = batch_capture(b);
         if (rc) return fail(nullptr, rc, b->ctx[0]->err);
