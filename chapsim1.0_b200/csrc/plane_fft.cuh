@@ -7,7 +7,7 @@
 // The chained form (k_div_fftx, k_fftz<-1>, ..., k_fftz<+1>, k_fftx_inv)
 // moves the spectrum through HBM between the x and the z transforms.  Here
 // one block owns a whole row j:
-//   k_div_fft2  DIVG_tg for the x-z plane of row j (in FP32 RHSLLPHI too),
+//   k_div_fft2  DIVG_tg for the x-z plane of row j (RHSLLPHI written once),
 //               x transform of z-line pairs (two real lines k = 2p, 2p+1
 //               packed into one complex line), unpacking into z lines of the
 //               half spectrum, z transform, spectrum of row j written once;
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__((p2_nt<SpecT<R>, NX1 * NX2 * NZ1 * NZ2>()), 1)
         const double w = W[c], wp = W[pidx(g, i, j, wrapp(k, N))];
         const double dv = (up - u) * coe1 + (vp - v) * coe2 + (wp - w) * g.dzi;
         const double val = dv * coe0;
-        if constexpr (sizeof(R) == 4) RHSLL[iidx(g, i, j, k)] = (R)val;  // FP64: see k_correct
+        RHSLL[iidx(g, i, j, k)] = (R)val;
         C* line = smc + (k >> 1) * LDX;
         if ((k & 1) == 0) line[i].x = (T)val; else line[i].y = (T)val;
     }

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(p2c_nt<SpecT<R>>(), 1) k_div_fft2c(Geo g, cons
                 out[e] = (R)x;
                 val[part][e] = (T)x;
             }
-            if constexpr (sizeof(R) == 4) st16(RHSLL + iidx(g, i0, j, k), out);  // FP64: see k_correct
+            st16(RHSLL + iidx(g, i0, j, k), out);
         }
         C* line = xb + pair * LDX + i0;
 #pragma unroll
