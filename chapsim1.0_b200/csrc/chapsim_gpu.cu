@@ -2066,13 +2066,14 @@ int chapsim_advance_xinout(chapsim_ctx_t* io, int32_t nsteps, double dt0, double
         for (int ns = 1; ns <= 3; ++ns) launch_xio_pair_substep(io, ns);
     }
     CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(tg->stream));
+    // Each check waits for its domain's stream and clears its error word.  Both, before the TG domain's error is
+    // returned: the TG stream waits for the main domain's inlet reads only, not for the rest of its substeps.
     rc = check_device_error(tg);
+    const int rc_io = check_device_error(io);
     if (rc) return fail(io, rc, "TG domain: " + tg->err);
-    rc = check_device_error(io);
     if (dt_out) *dt_out = io->st_host->dt;
     if (cfl_out) *cfl_out = io->st_host->cflmm;
-    return rc;
+    return rc_io;
 }
 
 int chapsim_xinout_thermal_inlet(chapsim_ctx_t* ctx, const double* state7) {
