@@ -2162,8 +2162,15 @@ int chapsim_launch_count(const chapsim_ctx_t* ctx, uint64_t* count) {
 
 int chapsim_kernels_per_step(const chapsim_ctx_t* ctx, int32_t* count) {
     if (!ctx || !count) return CHAPSIM_ERR_BADARG;
-    int per = 2 + 3 * (ctx->thermal ? 15 : 9 + (ctx->k1_kind == 1 ? 1 : 0));
-    *count = per;
+    // per substep; the step start launches the CFL numbers and the dt rule (and the pair's, with inflow)
+    int sub;
+    if (ctx->domain == 1)  // right-hand side (with its own x sweep in the split form), sweeps, Poisson solve, correction
+        sub = 4 + (ctx->k1_kind == 1 ? 1 : 0) + (ctx->plane_kind == 1 ? 3 : 5);
+    else if (ctx->domain == 2)
+        sub = (ctx->ivis ? 10 : ctx->prec == CHAPSIM_PREC_MIXED ? 9 : 8) + (ctx->thermal ? 4 : 0);
+    else
+        sub = 12 + (ctx->thermal ? 7 : 0);
+    *count = (ctx->domain == 3 ? 3 : 2) + 3 * sub;
     return CHAPSIM_OK;
 }
 

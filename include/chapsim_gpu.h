@@ -571,7 +571,8 @@ int chapsim_sync(chapsim_ctx_t* ctx);
  * each kernel node). */
 int chapsim_launch_count(const chapsim_ctx_t* ctx, uint64_t* count);
 
-/* Kernels launched per call of chapsim_advance_tg per step (for accounting). */
+/* Kernels that one step of chapsim_advance_tg (of chapsim_advance_xinout, the
+ * TG domain's own not among them) launches with the present settings. */
 int chapsim_kernels_per_step(const chapsim_ctx_t* ctx, int32_t* count);
 
 #ifdef __cplusplus
