@@ -37,7 +37,7 @@ EXPORTED = ["chapsim_gpu_init", "chapsim_gpu_finalize", "chapsim_last_error_stri
             "chapsim_prop_table_init", "chapsim_therm_prop_update_points", "chapsim_thermal_init",
             "chapsim_download_thermal_fields", "chapsim_mlp_init", "chapsim_mlp_set_params", "chapsim_mlp_get_params",
             "chapsim_mlp_gradients", "chapsim_mlp_train", "chapsim_mlp_infer_points", "chapsim_thermal_use_mlp",
-            "chapsim_mlp_judge", "chapsim_autotune", "chapsim_batch_create", "chapsim_batch_advance",
+            "chapsim_mlp_judge", "chapsim_autotune", "chapsim_get_choice", "chapsim_batch_create", "chapsim_batch_advance",
             "chapsim_set_buoyancy", "chapsim_upload_weighted_pressure",
             "chapsim_batch_get_stream", "chapsim_batch_destroy", "chapsim_pp_mean_zx_tg", "chapsim_pp_mean_t_tg",
             "chapsim_pp_monitor_tg", "chapsim_download_pp_means_tg", "chapsim_upload_pp_means_tg", "chapsim_divgck_io",
@@ -178,6 +178,7 @@ def load_library(path: str = LIB_PATH):
     L.chapsim_mlp_infer_points.argtypes = [vp, ctypes.c_int64] + [_dp] * 7
     L.chapsim_thermal_use_mlp.argtypes = [vp, ctypes.c_int32]
     L.chapsim_mlp_judge.argtypes = [vp, _dp]
+    L.chapsim_get_choice.argtypes = [vp, ctypes.POINTER(ctypes.c_int32)]
     L.chapsim_autotune.argtypes = [vp, ctypes.c_int32, ctypes.POINTER(ctypes.c_int32), ctypes.POINTER(ctypes.c_float)]
     L.chapsim_divgck_io.argtypes = [vp, ctypes.POINTER(ctypes.c_double)]
     i32 = ctypes.c_int32
@@ -313,10 +314,6 @@ class ChannelTG:
         domain (0 explicit, 1 Crank-Nicolson); the TG domain accepts 0 only.
         pdl: launch the step's kernels with programmatic dependent launch."""
         self.lib = load_library()
-        # variant bits in use (chapsim_autotune): what the library starts with
-        self.choice = 0
-        if precision == "fp64" and self.IDOMAIN == 1:
-            self.choice = 64 | 256 | (6 if setup.L >= 192 else 4 if setup.L >= 64 else 0)
         if precision not in PRECISIONS:
             raise ValueError(f"precision must be one of {sorted(PRECISIONS)}")
         self.precision = precision
@@ -350,6 +347,9 @@ class ChannelTG:
         if rc != 0:
             raise ChapsimError(rc, self.lib.chapsim_last_error_string(None).decode())
         self.h = h
+        ch = ctypes.c_int32()
+        self._check(self.lib.chapsim_get_choice(h, ctypes.byref(ch)))
+        self.choice = ch.value  # variant bits in use (autotune): what the library starts with
 
     @classmethod
     def create(cls, L, M, N, HX, HZ, STR2, REN, iFlowDriven=1, Cf_Given=8.18e-3, **kw):
@@ -638,7 +638,8 @@ class ChannelTG:
         transforms; bit 4: two-way y-solve; bit 5: sequential y-solve with its
         forward intermediate in shared memory at one block per SM; bit 6: warp
         affine scans over the sequential factors; bit 8: z-sweep tiles of 16
-        lines instead of 32; bits 9-12: kept as forced, no effect); returns
+        lines instead of 32; bits 10 and 11: lines in pairs in the z and y sweeps,
+        without effect in FP64; bits 9 and 12: kept as forced, no effect); returns
         (choice bits, {variant: ms})."""
         ch = ctypes.c_int32()
         ms = (ctypes.c_float * 19)()

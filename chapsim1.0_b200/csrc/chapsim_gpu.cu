@@ -2757,6 +2757,23 @@ extern "C" int chapsim_mlp_judge(chapsim_ctx_t* ctx, double* max_rel_err) {
 }
 
 // ----------------------------- autotuner -----------------------------------
+namespace {
+// the kernel variants in use, in chapsim_autotune's bit form; the main domains have the y-solve's only
+int variant_bits(const chapsim_ctx* ctx) {
+    const int k = ctx->ysolve_kind;
+    const int y = (k == 1 ? 1 : 0) | (k == 2 ? 16 : 0) | (k == 3 ? 32 : 0) | (k == 4 ? 64 : 0);
+    if (ctx->domain != 1) return y;
+    return y | (ctx->k1_kind << 1) | (ctx->plane_kind << 3) | (ctx->zs_tw == 16 ? 256 : 0) | (ctx->fz_pipe ? 512 : 0) |
+           (ctx->zs_il == 2 ? 1024 : 0) | (ctx->ys_il == 2 ? 2048 : 0) | (ctx->fz_prefetch ? 4096 : 0);
+}
+}  // namespace
+
+extern "C" int chapsim_get_choice(const chapsim_ctx_t* ctx, int32_t* choice) {
+    if (!ctx || !choice) return CHAPSIM_ERR_BADARG;
+    *choice = variant_bits(ctx);
+    return CHAPSIM_OK;
+}
+
 // Times the Poisson y-solve variants (warp Thomas/PCR hybrid, sequential
 // Thomas, two-way, sequential at one block per SM, warp scans) on this
 // context's grid and keeps the fastest.  The spectral array is scratch
@@ -3019,11 +3036,7 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    if (choice)
-        *choice = (ctx->ysolve_kind == 1 ? 1 : 0) | (ctx->k1_kind << 1) | (ctx->plane_kind << 3) |
-                  (ctx->ysolve_kind == 2 ? 16 : 0) | (ctx->ysolve_kind == 3 ? 32 : 0) | (ctx->ysolve_kind == 4 ? 64 : 0) |
-                  (ctx->zs_tw == 16 ? 256 : 0) | (ctx->fz_pipe ? 512 : 0) | (ctx->zs_il == 2 ? 1024 : 0) |
-                  (ctx->ys_il == 2 ? 2048 : 0) | (ctx->fz_prefetch ? 4096 : 0);
+    if (choice) *choice = variant_bits(ctx);
     if (ms) {
         ms[0] = t[0]; ms[1] = t[1]; ms[2] = tk[0]; ms[3] = tk[1]; ms[4] = tk[2];
         ms[5] = tp[0]; ms[6] = tp[1]; ms[7] = t[2]; ms[8] = t[3]; ms[9] = t[4];

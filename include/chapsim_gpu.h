@@ -535,6 +535,10 @@ int chapsim_dump_write(chapsim_ctx_t* ctx, const char* path_prefix, int32_t iter
  * with right-hand side 0 (L = 32), 2 (64 to 128) or 3 (longer lines). */
 int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choice, float* ms);
 
+/* The setting in use, in the bit form of chapsim_autotune: before that call what
+ * the context started with.  Main-domain contexts have bits 0 and 4 to 6. */
+int chapsim_get_choice(const chapsim_ctx_t* ctx, int32_t* choice);
+
 /* An ensemble of independent periodic channels (any grids and precisions, one
  * device) advanced together: one CUDA graph per step holds every member's
  * kernels as parallel branches, so small members fill the GPU together.

@@ -73,3 +73,31 @@ def test_kernels_per_step_xinout(thermal):
     assert io.launch_count() - before == 2 * io.kernels_per_step()
     io.close()
     tg.close()
+
+
+@pytest.mark.parametrize("kind,shape,precision", [
+    ("tg", (32, 32, 32), "fp64"), ("tg", (64, 32, 32), "fp64"), ("tg", (128, 32, 64), "fp64"), ("tg", (192, 32, 32), "fp64"),
+    ("tg", (64, 32, 32), "mixed"), ("io", (64, 32, 32), "fp64"), ("io", (32, 32, 192), "fp64"), ("io", (64, 32, 32), "mixed")])
+def test_starting_choice_is_what_runs(kind, shape, precision):
+    """Forcing the choice that a new context names changes no bit of its fields."""
+    make = _tg if kind == "tg" else _io
+    a = make(*shape, precision=precision)
+    b = make(*shape, precision=precision, force=a.choice)
+    assert b.choice == a.choice
+    for c in (a, b):
+        c.advance(3, DT, 1e-6, 0.5)
+    get = (lambda c: c.download()) if kind == "tg" else (lambda c: c.download_io())
+    for x, y in zip(get(a), get(b)):
+        assert np.array_equal(x, y)
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("shape", [(32, 32, 32), (32, 32, 384)])
+def test_main_domain_keeps_a_forced_choice(shape):
+    """The bits of the periodic channel's kernels stay clear in a main-domain context."""
+    c = _io(*shape)
+    assert c.choice & ~(1 | 16 | 32 | 64) == 0
+    for force in (0, 1, 16, 64):
+        assert c.autotune(force=force)[0] == force
+    c.close()
