@@ -2298,11 +2298,16 @@ extern "C" int chapsim_prop_table_init(chapsim_ctx_t* ctx, const chapsim_prop_ta
     }
     CK(cudaSetDevice(ctx->device));
     CK(cudaStreamSynchronize(ctx->stream));
-    cudaFree(ctx->ptab);
-    ctx->ptab = nullptr;
     const size_t rbytes = rows.size() * sizeof(SplineRow);
     const size_t kbytes = (size_t)2 * n * sizeof(double);
-    CK(cudaMalloc(&ctx->ptab, rbytes + kbytes));
+    void* ptab = nullptr;  // the old table stays when there is no room for the new one
+    CK(cudaMalloc(&ptab, rbytes + kbytes));
+    if (int rc = drop_step_graph(ctx)) {
+        cudaFree(ptab);
+        return rc;
+    }
+    cudaFree(ctx->ptab);
+    ctx->ptab = ptab;
     if (!ctx->pstat) CK(cudaMalloc(&ctx->pstat, sizeof(PropStatus)));
     char* base = static_cast<char*>(ctx->ptab);
     double* keys = reinterpret_cast<double*>(base + rbytes);
@@ -2585,6 +2590,7 @@ extern "C" int chapsim_mlp_init(chapsim_ctx_t* ctx, double dh_lo, double dh_hi, 
         nm.off[k] = 0.5f * (lo + hi);
         nm.scale[k] = fmaxf(0.5f * (hi - lo), 1e-6f);
     }
+    if (int rc = drop_step_graph(ctx)) return rc;  // it holds the normalisation
     ctx->mlp_norm = nm;
     // Glorot-uniform weights from a SplitMix64 stream, zero biases
     std::vector<float> p(MLP_NPARAM, 0.f);

@@ -5,7 +5,7 @@ import math
 import numpy as np
 import pytest
 
-from chapsim import gpu
+from chapsim import gpu, thermo
 from chapsim.mesh import channel_setup
 from chapsim.fields import initial_field
 
@@ -44,3 +44,44 @@ def test_ensemble_follows_its_members_settings(force):
     e.close()
     for c in solo + grp:
         c.close()
+
+
+def _heated(seed=63):
+    L = M = N = 32
+    s = channel_setup(L, M, N, 2 * math.pi, math.pi, 2.0, 2800.0)
+    Q, PR = initial_field(s, seed, 0.1)
+    rows, T0 = thermo.synthetic_table()
+    tab = thermo.SplineTable.from_rows(rows, T0)
+    c = gpu.ChannelIO(s, ivisscheme=gpu.VIS_IMPLICIT)
+    ones = np.ones(c.field_shape())
+    c.upload_io(Q, PR, ones, ones, ones)
+    DH = np.zeros(c.field_shape())
+    DH[:, 1:M + 1] = 1e-3 * np.random.default_rng(seed).uniform(-1.0, 1.0, (N, M, L))
+    c.thermal_init(tab, DH, 0.5, 0.5, 1.0 / 2800.0 / (tab.ref["M0"] * tab.ref["CP0"] / tab.ref["K0"]))
+    c.set_dt(1e-3)
+    return c, tab
+
+
+@pytest.mark.parametrize("what", ["table", "mlp"])
+def test_new_property_source_reaches_the_captured_step(what):
+    """A second property table, or a model of another range, after the first captured step.  The second context is told
+    a setting that it already has besides, which asks for a new capture by itself."""
+    out = []
+    for again in (False, True):
+        c, tab = _heated()
+        lo, hi = float(tab.lists["DH"][0]), float(tab.lists["DH"][-1])
+        if what == "mlp":
+            c.mlp_init(lo + 0.02 * (hi - lo), hi - 0.02 * (hi - lo), seed=5)
+            c.thermal_use_mlp(True)
+        c.advance(1, 1e-3, 1e-6, 0.5)
+        if what == "table":
+            c.prop_table_init(tab, fix_swap=True)
+        else:
+            c.mlp_init(lo + 0.2 * (hi - lo), hi - 0.2 * (hi - lo), seed=5)
+        if again:
+            c.set_buoyancy(0, 0.0)
+        c.advance(2, 1e-3, 1e-6, 0.5)
+        out.append(list(c.download_io()) + list(c.download_thermal().values()))
+        c.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
