@@ -1238,16 +1238,6 @@ int chapsim_gpu_init(const chapsim_grid_t* grid, const chapsim_coefs_t* cf, cons
     g.yz = ctx->yz;
     k_ysolve_zero_factors<<<1, 32, 0, ctx->stream>>>(g, ctx->yz);
     INIT_CK(cudaGetLastError());
-    if (ctx->prec == CHAPSIM_PREC_FP64 && !xio) {
-        // FP64 contexts start with the y-solve by affine scans: faster than the others at every size measured
-        // (warp hybrid / scans in registers: 43 / 14 us at 128^3, 74 / 22 at 192 x 128 x 192, 449 / 133 at
-        // 384 x 256 x 384).  Mixed-precision contexts start with the hybrid: their FP32 fields
-        // are reproduced to the bit.
-        INIT_CK(cudaMalloc(&ctx->YF3, (size_t)g.LH * M * N * sizeof(double)));
-        ysolve_scan_factors(ctx);
-        INIT_CK(cudaGetLastError());
-        ctx->ysolve_kind = 4;
-    }
     // fields
     INIT_CK(cudaMalloc(&ctx->Q, (size_t)(3 * g.FS) * sizeof(double)));
     INIT_CK(cudaMalloc(&ctx->PR, (size_t)g.FS * sizeof(double)));
@@ -1367,6 +1357,21 @@ int chapsim_gpu_init(const chapsim_grid_t* grid, const chapsim_coefs_t* cf, cons
         g_init_error = ctx->err;
         chapsim_gpu_finalize(ctx);
         return rc;
+    }
+    if (ctx->prec == CHAPSIM_PREC_FP64 && !xio) {
+        // FP64 contexts start with the y-solve by affine scans: faster than the others at every size measured
+        // (warp hybrid / scans in registers: 43 / 14 us at 128^3, 74 / 22 at 192 x 128 x 192, 449 / 133 at
+        // 384 x 256 x 384).  Mixed-precision contexts start with the hybrid: their FP32 fields
+        // are reproduced to the bit.  Last, as the only table that a context can do without: where the pivots
+        // do not fit beside the fields, the hybrid, which reads none, stays.
+        if (cudaMalloc(&ctx->YF3, (size_t)g.LH * M * N * sizeof(double)) == cudaSuccess) {
+            ysolve_scan_factors(ctx);
+            INIT_CK(cudaGetLastError());
+            ctx->ysolve_kind = 4;
+        } else {
+            ctx->YF3 = nullptr;
+            cudaGetLastError();
+        }
     }
 
 #undef INIT_CK
