@@ -290,8 +290,8 @@ std::vector<double2> twiddles(int n) {
 }
 
 template <typename R> size_t smem_rhs(const Geo& g) { return (size_t)(RHS_WPB * 3 * (g.L + 33)) * sizeof(R); }
-template <typename R> size_t smem_z(const Geo& g, int tw) { return (size_t)(2 * tw * (g.N + 33)) * sizeof(R); }
-template <typename R> size_t smem_y(const Geo& g) { return (size_t)(32 * (g.M + 33)) * sizeof(R); }
+size_t smem_z(const Geo& g, int tw) { return (size_t)(2 * tw * (g.N + 33)) * sizeof(float); }
+size_t smem_y(const Geo& g) { return (size_t)(32 * (g.M + 33)) * sizeof(float); }
 template <typename R> size_t smem_xs(const Geo& g) { return (size_t)((XS_NT / 32) * (g.L + 33)) * sizeof(R); }
 template <typename R> size_t smem_rt() { return (size_t)(RT_SLOTS * RT_SLOT) * sizeof(R); }
 // planes per k-chunk of the 2.5D right-hand-side kernel: enough blocks to fill
@@ -501,12 +501,12 @@ int configure_momentum(chapsim_ctx* ctx) {
     DISPATCH_S(g.L / 32, ctx->rb_nw = rb_warps<R>(g.L, bulk_smem_limit(k_rhs_xsweep_bulk<S, R>)));
     if (ctx->rb_nw > 0) DISPATCH_S(g.L / 32, CK(set_smem(k_rhs_xsweep_bulk<S, R>, rb_smem<R>(g.L, ctx->rb_nw))));
     if constexpr (sizeof(R) == 4) {
-        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 32, 1>, smem_z<R>(g, 32))));
-        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 16, 1>, smem_z<R>(g, 16))));
-        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 32, 2>, smem_z<R>(g, 32))));
-        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, R, 16, 2>, smem_z<R>(g, 16))));
-        DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, R, 1>, smem_y<R>(g))));
-        DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, R, 2>, smem_y<R>(g))));
+        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, 32, 1>, smem_z(g, 32))));
+        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, 16, 1>, smem_z(g, 16))));
+        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, 32, 2>, smem_z(g, 32))));
+        DISPATCH_S(g.N / 32, CK(set_smem(k_zsweep<S, 16, 2>, smem_z(g, 16))));
+        DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, 1>, smem_y(g))));
+        DISPATCH_S(g.M / 32, CK(set_smem(k_ysweep<S, 2>, smem_y(g))));
     }
     DISPATCH_S(g.L / 32, CK(set_smem(k_xsweep<S, R>, smem_xs<R>(g))));
     CK(set_smem(k_rhs_point<R>, smem_rt<R>()));
@@ -685,21 +685,20 @@ void launch_zsweep(chapsim_ctx* ctx, const StepFields<double>& f, const double* 
     }
 }
 void launch_zsweep(chapsim_ctx* ctx, const StepFields<float>& f, const float* fac) {
-    using R = float;
     const Geo& g = ctx->g;
     const int tw = ctx->zs_tw;
-    const size_t sz = smem_z<R>(g, tw);
-    const int zb_want = g.N / 32 <= 4 ? 3 : 2;  // zsweep_blocks<R, S>
+    const size_t sz = smem_z(g, tw);
+    const int zb_want = g.N / 32 <= 4 ? 3 : 2;  // zsweep_blocks<S>
     const int zb = sz * zb_want <= 226 * 1024 ? zb_want : (sz <= 113 * 1024 ? 2 : 1);
     const int nz = std::min((g.L / tw) * (3 * g.M - 1), zb * ctx->nsm);
     if (tw == 16 && ctx->zs_il == 2) {
-        DISPATCH_S(g.N / 32, (launch_pdl(ctx->pdl, k_zsweep<S, R, 16, 2>, nz, SWEEP_NT, sz, ctx->stream, g, f.RHS, fac)));
+        DISPATCH_S(g.N / 32, (launch_pdl(ctx->pdl, k_zsweep<S, 16, 2>, nz, SWEEP_NT, sz, ctx->stream, g, f.RHS, fac)));
     } else if (tw == 16) {
-        DISPATCH_S(g.N / 32, (launch_pdl(ctx->pdl, k_zsweep<S, R, 16, 1>, nz, SWEEP_NT, sz, ctx->stream, g, f.RHS, fac)));
+        DISPATCH_S(g.N / 32, (launch_pdl(ctx->pdl, k_zsweep<S, 16, 1>, nz, SWEEP_NT, sz, ctx->stream, g, f.RHS, fac)));
     } else if (ctx->zs_il == 2) {
-        DISPATCH_S(g.N / 32, (launch_pdl(ctx->pdl, k_zsweep<S, R, 32, 2>, nz, SWEEP_NT, sz, ctx->stream, g, f.RHS, fac)));
+        DISPATCH_S(g.N / 32, (launch_pdl(ctx->pdl, k_zsweep<S, 32, 2>, nz, SWEEP_NT, sz, ctx->stream, g, f.RHS, fac)));
     } else {
-        DISPATCH_S(g.N / 32, (launch_pdl(ctx->pdl, k_zsweep<S, R, 32, 1>, nz, SWEEP_NT, sz, ctx->stream, g, f.RHS, fac)));
+        DISPATCH_S(g.N / 32, (launch_pdl(ctx->pdl, k_zsweep<S, 32, 1>, nz, SWEEP_NT, sz, ctx->stream, g, f.RHS, fac)));
     }
 }
 
@@ -712,14 +711,13 @@ void launch_ysweep(chapsim_ctx* ctx, const StepFields<double>& f, const double* 
                                   16 * (NSEG * SR / yseg_rows(NSEG * SR)), 0, ctx->stream, g, f.Q, f.RHS, ctx->st, fac, ns)));
 }
 void launch_ysweep(chapsim_ctx* ctx, const StepFields<float>& f, const float* fac, int ns) {
-    using R = float;
     const Geo& g = ctx->g;
     dim3 gry(g.L / 32, g.N, 2);  // layer 0: u then v, layer 1: w
     if (ctx->ys_il == 2) {
-        DISPATCH_S(g.M / 32, (launch_pdl(ctx->pdl, k_ysweep<S, R, 2>, gry, SWEEP_NT, smem_y<R>(g), ctx->stream, g, f.Q, f.RHS,
+        DISPATCH_S(g.M / 32, (launch_pdl(ctx->pdl, k_ysweep<S, 2>, gry, SWEEP_NT, smem_y(g), ctx->stream, g, f.Q, f.RHS,
                                          ctx->st, fac, ns)));
     } else {
-        DISPATCH_S(g.M / 32, (launch_pdl(ctx->pdl, k_ysweep<S, R, 1>, gry, SWEEP_NT, smem_y<R>(g), ctx->stream, g, f.Q, f.RHS,
+        DISPATCH_S(g.M / 32, (launch_pdl(ctx->pdl, k_ysweep<S, 1>, gry, SWEEP_NT, smem_y(g), ctx->stream, g, f.Q, f.RHS,
                                          ctx->st, fac, ns)));
     }
 }
@@ -1266,10 +1264,8 @@ int chapsim_gpu_init(const chapsim_grid_t* grid, const chapsim_coefs_t* cf, cons
         INIT_CK(cudaMalloc(&f.MU, (size_t)g.FS * sizeof(double)));
         INIT_CK(cudaMalloc(&f.DST, (size_t)(3 * g.FS) * sizeof(double)));
         INIT_CK(cudaMalloc(&f.MST, (size_t)(3 * g.FS) * sizeof(double)));
-        INIT_CK(cudaMalloc(&f.DIVU, (size_t)g.FS * sizeof(double)));
         INIT_CK(cudaMemset(f.G, 0, (size_t)(3 * g.FS) * sizeof(double)));
         INIT_CK(cudaMemset(f.EX0, 0, (size_t)(3 * g.FI) * sizeof(double)));
-        INIT_CK(cudaMemset(f.DIVU, 0, (size_t)g.FS * sizeof(double)));
         k_fill<<<4 * nsm, XIO_NT, 0, ctx->stream>>>(f.DST, 3 * g.FS, 1.0);  // src/MEMALLOCT.f90:200-201
         k_fill<<<4 * nsm, XIO_NT, 0, ctx->stream>>>(f.MST, 3 * g.FS, 1.0);
         INIT_CK(cudaGetLastError());
@@ -1390,7 +1386,7 @@ void chapsim_gpu_finalize(chapsim_ctx_t* ctx) {
     cudaFree(ctx->pp_inst); cudaFree(ctx->pp_avg); cudaFree(ctx->pp_part); cudaFree(ctx->pp_mon);
     cudaFree(ctx->ppio_set); cudaFree(ctx->ppio_part);
     cudaFree(ctx->io.G); cudaFree(ctx->io.EX0); cudaFree(ctx->io.RHO); cudaFree(ctx->io.MU0); cudaFree(ctx->io.MU);
-    cudaFree(ctx->io.DST); cudaFree(ctx->io.MST); cudaFree(ctx->io.DIVU);
+    cudaFree(ctx->io.DST); cudaFree(ctx->io.MST);
     cudaFree(ctx->iof.G); cudaFree(ctx->iof.EX0); cudaFree(ctx->iof.DST); cudaFree(ctx->iof.MST); cudaFree(ctx->iof.DIVU);
     cudaFree(const_cast<double*>(ctx->io.PR0A));
     cudaFree(ctx->ptab); cudaFree(ctx->pstat); cudaFree(ctx->pbuf);

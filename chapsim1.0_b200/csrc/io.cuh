@@ -31,7 +31,7 @@
 // PR0A/PR0B: PR0_io(:,:,:,1) and PR0_io(:,:,:,2) of iWeightedPre = 1 (NULL when
 // off).  igrav/fa: iGravity and F_A of thermal_gravity (src/Flow_State.f90:95-125).
 // F is the storage type of the flow fields G, Q, PR, EXPLT0, RHS, D_STG, MU_STG
-// and DivU: double, or float in the mixed-precision step.  The property
+// and DivU (NULL in FP64, whose right-hand side forms it): double, or float in the mixed-precision step.  The property
 // fields (DENSITY, DENSITY0, Viscousity, Viscousity0) stay FP64 (they come
 // from the FP64 property update), and the kernels evaluate in FP64.
 template <typename F>

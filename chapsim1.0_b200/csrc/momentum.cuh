@@ -629,14 +629,15 @@ __global__ void __launch_bounds__(RHS_WPB * 32, RHS_MINB_P(R, PV)) k_rhs_xsweep(
     }
 }
 
-// Resident blocks per SM of the persistent z sweep: 3 for FP32 lines up to
+// The staged z and y sweeps: FP32 only (FP64 lines are solved in registers, k_zsweep_reg and k_ysweep_reg).
+// Resident blocks per SM of the persistent z sweep: 3 for lines up to
 // 128 (80 registers; the two tile buffers take 41 KB), else 2 (128
-// registers; longer FP32 lines would spill under the tighter budget, and
+// registers; longer lines would spill under the tighter budget, and
 // their buffers leave room for two blocks only).
-template <typename R, int S> __host__ __device__ constexpr int zsweep_blocks() { return sizeof(R) == 4 && S <= 4 ? 3 : 2; }
+template <int S> __host__ __device__ constexpr int zsweep_blocks() { return S <= 4 ? 3 : 2; }
 // Lines (consecutive i) per tile, TW: 32 or 16 (autotuned, chapsim_autotune bit 8).  16 halves the
-// two tile buffers (2 x 32 x (N + 33) doubles are 213 KB at N = 384: one block per SM) and each z
-// position of a tile still reads whole 32-byte sectors (64 or 128 bytes per row segment).
+// two tile buffers (2 x 32 x (N + 33) words are 107 KB at N = 384) and each z position of a tile still
+// reads whole 32-byte sectors (64 bytes per row segment).
 
 // ---------------------------------------------------------------------------
 // cyclic z sweep.  A tile is TW (32 or 16) consecutive i at fixed j, all
@@ -647,13 +648,14 @@ template <typename R, int S> __host__ __device__ constexpr int zsweep_blocks() {
 // Shared-memory layout of a tile: IL = 1 keeps each line contiguous (segment
 // padded, LS = N + 33 elements per line); IL = 2 interleaves the lines in
 // pairs, element z of line il at (il / 2) * 2 LS + 2 seg_pos(z) + il % 2, so
-// that one cp.async of two consecutive x points (8 bytes in FP32, 16 in FP64)
+// that one 8-byte cp.async of two consecutive x points
 // fills both lines of a pair: half the copy instructions, for 2-way bank
 // conflicts in the solve's segment reads (the lane stride is 2 (S + 1)).
 template <int IL> __device__ __forceinline__ int zs_line(int il, int LS) { return IL == 1 ? il * LS : (il >> 1) * 2 * LS + (il & 1); }
 
-template <int S, typename R, int TW, int IL>
-__global__ void __launch_bounds__(SWEEP_NT, (zsweep_blocks<R, S>())) k_zsweep(Geo g, R* __restrict__ RHS, const R* __restrict__ fac) {
+template <int S, int TW, int IL>
+__global__ void __launch_bounds__(SWEEP_NT, zsweep_blocks<S>()) k_zsweep(Geo g, float* __restrict__ RHS, const float* __restrict__ fac) {
+    using R = float;
     pdl_wait();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     R* smb = reinterpret_cast<R*>(sm_raw);
@@ -686,8 +688,7 @@ __global__ void __launch_bounds__(SWEEP_NT, (zsweep_blocks<R, S>())) k_zsweep(Ge
             } else {
                 R* dst = buf + c * 2 * LS + 2 * seg_pos<S>(z);
                 const R* src = Rz + 2 * c + ks * z;
-                if constexpr (sizeof(R) == 8) cp_async16(dst, src);
-                else cp_async8(reinterpret_cast<double*>(dst), reinterpret_cast<const double*>(src));
+                cp_async8(reinterpret_cast<double*>(dst), reinterpret_cast<const double*>(src));
             }
         }
     };
@@ -807,10 +808,11 @@ __global__ void __launch_bounds__(TI * NSEG, zr_minb<SR>(TI * NSEG)) k_zsweep_re
 // work into about four component times instead of six.
 // IL: the tile layout of k_zsweep (1 lines contiguous, 2 interleaved in pairs: one copy and one
 // vector access of Q per two x points).
-template <int S, typename R, int IL>
-__global__ void __launch_bounds__(SWEEP_NT, (S >= 6 ? 2 : (sizeof(R) == 4 ? 4 : 3))) k_ysweep(Geo g, R* __restrict__ Q, const R* __restrict__ RHS,
-                                                     const DevState* __restrict__ st, const R* __restrict__ fac,
+template <int S, int IL>
+__global__ void __launch_bounds__(SWEEP_NT, (S >= 6 ? 2 : 4)) k_ysweep(Geo g, float* __restrict__ Q, const float* __restrict__ RHS,
+                                                     const DevState* __restrict__ st, const float* __restrict__ fac,
                                                      int ns) {
+    using R = float;
     pdl_wait();
     extern __shared__ __align__(16) unsigned char sm_raw[];
     R* sm = reinterpret_cast<R*>(sm_raw);
@@ -842,8 +844,7 @@ __global__ void __launch_bounds__(SWEEP_NT, (S >= 6 ? 2 : (sizeof(R) == 4 ? 4 : 
             } else {
                 R* dst = sm + c * 2 * LS + 2 * seg_pos<S>(jl);
                 const R* src = Ry + 2 * c + js * jl;
-                if constexpr (sizeof(R) == 8) cp_async16(dst, src);
-                else cp_async8(reinterpret_cast<double*>(dst), reinterpret_cast<const double*>(src));
+                cp_async8(reinterpret_cast<double*>(dst), reinterpret_cast<const double*>(src));
             }
         }
         cp_async_wait_all();
