@@ -404,6 +404,7 @@ def kernel_bytes(L, precision="fp64"):
     CONVH0, RHS, RHSLLPHI, the spectrum and DPH are stored in 4-byte words."""
     w = 8.0 if precision == "fp64" else 4.0
     spec = 2.0 * (L // 2 + 1) / L * w  # complex spectrum, bytes per point
+    ll = 0.0 if precision == "fp64" else w  # RHSLLPHI, which the FP64 step does not store
     return {
         "k_cfl": 3 * w, "k_dt_factors": 0.0,
         "k_rhs_xsweep": 13 * w,            # Q x3, PR, H0 x3 in; H0 x3, RHS x3 out (x sweep in registers)
@@ -411,16 +412,16 @@ def kernel_bytes(L, precision="fp64"):
         "k_rhs_point+k_xsweep": 19 * w,    # the same, plus the RHS round trip of the separate x sweep
         "k_zsweep": 6 * w,                 # RHS x3 in/out
         "k_ysweep": 9 * w,                 # RHS x3, Q x3 in; Q x3 out
-        "k_div_fftx": 4 * w + spec,        # Q x3 in; RHSLLPHI, spectrum out
-        "k_div_fft2": 4 * w + spec,        # the same with the z transforms of the plane
-        "k_div_fft2c": 4 * w + spec,       # the same, the plane split over a thread-block cluster
+        "k_div_fftx": 3 * w + ll + spec,   # Q x3 in; RHSLLPHI (mixed), spectrum out
+        "k_div_fft2": 3 * w + ll + spec,   # the same with the z transforms of the plane
+        "k_div_fft2c": 3 * w + ll + spec,  # the same, the plane split over a thread-block cluster
         "k_fftz_fwd": 2 * spec, "k_fftz_inv": 2 * spec,
         "k_ysolve_warp": 2 * spec, "k_ysolve_seq": 2 * spec, "k_ysolve_2w": 2 * spec,
         "k_ysolve_scan": 2 * spec,         # the factors it reads are not algorithmic bytes
         "k_fftx_inv": spec + w,            # spectrum in; DPH out
         "k_fft2_inv": spec + w,            # the same with the inverse z transforms of the plane
         "k_fft2c_inv": spec + w,           # the same, the plane split over a thread-block cluster
-        "k_correct": 10 * w,               # DPH, Q x3, PR, RHSLLPHI in; Q x3, PR out
+        "k_correct": 9 * w + ll,           # DPH, Q x3, PR, RHSLLPHI (mixed) in; Q x3, PR out
     }
 
 

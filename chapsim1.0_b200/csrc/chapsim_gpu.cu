@@ -162,6 +162,7 @@ struct chapsim_ctx {
                                   // scans over the sequential factors (chapsim_autotune)
     int k1_kind = 0;              // 0: fused k_rhs_xsweep, 1: k_rhs_point + k_xsweep, 2: k_rhs_xsweep_bulk, 3: the wide
                                   // fused form, 16-byte loads (rhs_pv) (chapsim_autotune)
+    bool lap = false;             // RHSLLPHI of the FP64 pressure update is the Laplacian of DPH (lap_is_rhs)
     int plane_kind = 0;           // 0: chained x/z transforms, 1: fused plane transforms k_div_fft2/k_fft2_inv (chapsim_autotune)
     int zs_tw = 32;               // lines per tile of the z sweep, 32 or 16 (chapsim_autotune)
     int zs_il = 1;                // FP32 z-sweep tile layout: 1 line-contiguous, 2 lines interleaved in pairs (chapsim_autotune)
@@ -511,7 +512,8 @@ int configure_momentum(chapsim_ctx* ctx) {
     DISPATCH_S(g.L / 32, CK(set_smem(k_xsweep<S, R>, smem_xs<R>(g))));
     CK(set_smem(k_rhs_point<R>, smem_rt<R>()));
     using C = SpecT<R>;
-    DISPATCH_FFT(g.L, CK(set_smem(k_div_fftx<R, FN1, FN2>, smem_px<C>(g))));
+    DISPATCH_FFT(g.L, CK(set_smem(k_div_fftx<R, true, FN1, FN2>, smem_px<C>(g))));
+    if constexpr (sizeof(R) == 8) DISPATCH_FFT(g.L, CK(set_smem(k_div_fftx<R, false, FN1, FN2>, smem_px<C>(g))));
     DISPATCH_FFT(g.L, CK(set_smem(k_fftx_inv<FN1, FN2, C>, smem_px<C>(g))));
     DISPATCH_S(g.M / 32, CK(set_smem(k_ysolve_warp<S, C>, smem_yw<C>(g))));
     CK(set_smem(k_ysolve_seq<C, false>, smem_ysolve_seq(g.M, false)));
@@ -633,17 +635,18 @@ void launch_fftz(chapsim_ctx* ctx, C* sp, bool pdl) {
     DISPATCH_FFT(g.N, (launch_pdl(pdl, k_fftz<SIGN, FN1, FN2, C>, gfz, (fz_nt<C, FN1>()), smem_fz<C>(g), ctx->stream, g, sp)));
 }
 
-template <typename R>
-void launch_pressure(chapsim_ctx* ctx, const StepFields<R>& f, int ns) {
+// ST: the divergence kernels store RHSLLPHI (ctx->lap: k_correct does without).
+template <typename R, bool ST>
+void launch_pressure_t(chapsim_ctx* ctx, const StepFields<R>& f, int ns) {
     const Geo& g = ctx->g;
     cudaStream_t s = ctx->stream;
     using C = SpecT<R>;
     C* sp = spec<C>(ctx);
     if (ctx->plane_kind == 1) {
         if (ctx->p2c) {
-            P2C_DISPATCH(g.L, g.N, (plane_fft_cluster_fwd<R, XN1, XN2, ZN1, ZN2>(ctx->pdl, g, f.Q, f.RHSLL, sp, ctx->st, ns, s)));
+            P2C_DISPATCH(g.L, g.N, (plane_fft_cluster_fwd<R, ST, XN1, XN2, ZN1, ZN2>(ctx->pdl, g, f.Q, f.RHSLL, sp, ctx->st, ns, s)));
         } else {
-            P2_DISPATCH(g.L, g.N, (plane_fft_fwd<R, XN1, XN2, ZN1, ZN2>(ctx->pdl, g, f.Q, f.RHSLL, sp, ctx->st, ns, smem_p2<C>(g), s)));
+            P2_DISPATCH(g.L, g.N, (plane_fft_fwd<R, ST, XN1, XN2, ZN1, ZN2>(ctx->pdl, g, f.Q, f.RHSLL, sp, ctx->st, ns, smem_p2<C>(g), s)));
         }
         prof_mark(ctx);
         prof_mark(ctx);
@@ -660,7 +663,7 @@ void launch_pressure(chapsim_ctx* ctx, const StepFields<R>& f, int ns) {
         return;
     }
     dim3 grp((g.M + PX_TJ - 1) / PX_TJ, g.N);
-    DISPATCH_FFT(g.L, (launch_pdl(ctx->pdl, k_div_fftx<R, FN1, FN2>, grp, PX_NT, smem_px<C>(g), s, g, f.Q, f.RHSLL, sp, ctx->st, ns)));
+    DISPATCH_FFT(g.L, (launch_pdl(ctx->pdl, k_div_fftx<R, ST, FN1, FN2>, grp, PX_NT, smem_px<C>(g), s, g, f.Q, f.RHSLL, sp, ctx->st, ns)));
     prof_mark(ctx);
     launch_fftz<-1, C>(ctx, sp, ctx->pdl);
     prof_mark(ctx);
@@ -672,6 +675,23 @@ void launch_pressure(chapsim_ctx* ctx, const StepFields<R>& f, int ns) {
     prof_mark(ctx);
     ctx->launches += 5;
 }
+void launch_pressure(chapsim_ctx* ctx, const StepFields<double>& f, int ns) {
+    if (ctx->lap) launch_pressure_t<double, false>(ctx, f, ns);
+    else launch_pressure_t<double, true>(ctx, f, ns);
+}
+void launch_pressure(chapsim_ctx* ctx, const StepFields<float>& f, int ns) { launch_pressure_t<float, true>(ctx, f, ns); }
+template <typename R, bool LAP>
+void launch_correct(chapsim_ctx* ctx, const StepFields<R>& f, int ns) {
+    const Geo& g = ctx->g;
+    const long long tot = (long long)g.L * g.M * g.N / V16<R>::W;  // one thread per 16-byte group of an x line
+    launch_pdl(ctx->pdl, k_correct<R, LAP>, (int)((tot + CR_NT - 1) / CR_NT), CR_NT, 0, ctx->stream, g, f.Q, f.PR, dph<R>(ctx), f.RHSLL,
+               ctx->st, ns);
+}
+void launch_correct(chapsim_ctx* ctx, const StepFields<double>& f, int ns) {
+    if (ctx->lap) launch_correct<double, true>(ctx, f, ns);
+    else launch_correct<double, false>(ctx, f, ns);
+}
+void launch_correct(chapsim_ctx* ctx, const StepFields<float>& f, int ns) { launch_correct<float, false>(ctx, f, ns); }
 
 // Cyclic z sweep.  FP64: the register form, tiles of ctx->zs_tw lines.  FP32: persistent, as many
 // blocks as fit at once (two per SM where the two tile buffers allow).
@@ -739,9 +759,8 @@ void launch_substep_t(chapsim_ctx* ctx, int ns, bool factors) {
     prof_mark(ctx);
     launch_ysweep(ctx, f, fac, ns);
     prof_mark(ctx);
-    launch_pressure<R>(ctx, f, ns);
-    const long long tot = (long long)g.L * g.M * g.N / V16<R>::W;  // one thread per 16-byte group of an x line
-    launch_pdl(ctx->pdl, k_correct<R>, (int)((tot + CR_NT - 1) / CR_NT), CR_NT, 0, s, g, f.Q, f.PR, dph<R>(ctx), f.RHSLL, ctx->st, ns);
+    launch_pressure(ctx, f, ns);
+    launch_correct(ctx, f, ns);
     prof_mark(ctx);
     ctx->launches += 4;
 }
@@ -1101,6 +1120,35 @@ int build_step_graph(chapsim_ctx* ctx) {
 
 }  // namespace
 
+namespace {
+// True when the Poisson operator of the coefficients, applied to its solution, is the discrete Laplacian of k_correct
+// for every right-hand side that a divergence gives: the second difference's wavenumbers in x and z, and in y
+// a conservative operator with Neumann walls (its rows sum to zero, and its columns weighted by 1/DYFI: the pinned
+// row of the kx = kz = 0 mode then holds too).  The reference's set-up meets the bounds with a factor of two or more
+// to spare (measured over the seven lengths: 2^-50 DXQI, 2^-52, 2^-51); within them the two differ by no more
+// than the Laplacian's own rounding.
+bool lap_is_rhs(const chapsim_coefs_t& cf, int L, int M, int N) {
+    const double pi = 2.0 * std::asin(1.0), tol = std::ldexp(1.0, -49);
+    auto waves = [&](const double* ak, int n, double dqi) {
+        for (int i = 0; i < n; ++i) {
+            const double s = std::sin(pi * (double)std::min(i, n - i) / (double)n);
+            if (!(std::fabs(ak[i] - 4.0 * dqi * s * s) <= tol * dqi)) return false;
+        }
+        return true;
+    };
+    if (!waves(cf.ak1, L, cf.dxqi) || !waves(cf.ak3, N, cf.dzqi)) return false;
+    for (int j = 0; j < M; ++j) {
+        const double am = j > 0 ? cf.amph[j] : 0.0, ap = j < M - 1 ? cf.apph[j] : 0.0;
+        if (!(std::fabs(cf.acph[j] + (am + ap)) <= tol * std::fabs(cf.acph[j]))) return false;
+        if (j < M - 1) {
+            const double up = ap / cf.dyfi[j], dn = cf.amph[j + 1] / cf.dyfi[j + 1];
+            if (!(std::fabs(up - dn) <= tol * std::fabs(up))) return false;
+        }
+    }
+    return true;
+}
+}  // namespace
+
 // ============================== C ABI ========================================
 extern "C" {
 
@@ -1151,6 +1199,7 @@ int chapsim_gpu_init(const chapsim_grid_t* grid, const chapsim_coefs_t* cf, cons
     ctx->domain = grid->idomain;
     ctx->prec = prec;
     ctx->pdl = !(opts && opts->no_pdl);
+    ctx->lap = prec == CHAPSIM_PREC_FP64 && grid->idomain == 1 && lap_is_rhs(*cf, L, M, N);
     ctx->ivis = ivis;
     int rc;
 #define INIT_CK(call)                                  \
@@ -3010,8 +3059,8 @@ extern "C" int chapsim_autotune(chapsim_ctx_t* ctx, int32_t force, int32_t* choi
             if (kind == 1 && !p2) continue;
             ctx->plane_kind = kind;
             auto one = [&]() {
-                if (mixed) launch_pressure<float>(ctx, step_fields<float>(ctx), 1);
-                else launch_pressure<double>(ctx, step_fields<double>(ctx), 1);
+                if (mixed) launch_pressure(ctx, step_fields<float>(ctx), 1);
+                else launch_pressure(ctx, step_fields<double>(ctx), 1);
             };
             one();
             if (kind == 1 && ctx->p2c && cudaGetLastError() != cudaSuccess) {

@@ -7,7 +7,7 @@
 // The chained form (k_div_fftx, k_fftz<-1>, ..., k_fftz<+1>, k_fftx_inv)
 // moves the spectrum through HBM between the x and the z transforms.  Here
 // one block owns a whole row j:
-//   k_div_fft2  DIVG_tg for the x-z plane of row j (RHSLLPHI written once),
+//   k_div_fft2  DIVG_tg for the x-z plane of row j (RHSLLPHI too where k_correct reads it: ST),
 //               x transform of z-line pairs (two real lines k = 2p, 2p+1
 //               packed into one complex line), unpacking into z lines of the
 //               half spectrum, z transform, spectrum of row j written once;
@@ -43,7 +43,7 @@ __host__ __device__ inline int plane_fft_words(int L, int N) {
     return a > b ? a : b;
 }
 
-template <typename R, int NX1, int NX2, int NZ1, int NZ2>
+template <typename R, bool ST, int NX1, int NX2, int NZ1, int NZ2>
 __global__ void __launch_bounds__((p2_nt<SpecT<R>, NX1 * NX2 * NZ1 * NZ2>()), 1) k_div_fft2(Geo g, const R* __restrict__ Q, R* __restrict__ RHSLL,
                                                        SpecT<R>* __restrict__ SP, const DevState* __restrict__ st,
                                                        int ns) {
@@ -74,7 +74,7 @@ __global__ void __launch_bounds__((p2_nt<SpecT<R>, NX1 * NX2 * NZ1 * NZ2>()), 1)
         const double w = W[c], wp = W[pidx(g, i, j, wrapp(k, N))];
         const double dv = (up - u) * coe1 + (vp - v) * coe2 + (wp - w) * g.dzi;
         const double val = dv * coe0;
-        RHSLL[iidx(g, i, j, k)] = (R)val;
+        if constexpr (ST) RHSLL[iidx(g, i, j, k)] = (R)val;
         C* line = smc + (k >> 1) * LDX;
         if ((k & 1) == 0) line[i].x = (T)val; else line[i].y = (T)val;
     }
@@ -205,17 +205,19 @@ template <typename R, int XN1, int XN2, int ZN1, int ZN2>
 cudaError_t plane_fft_attrs(cudaError_t (*set)(const void*, size_t), size_t bytes) {
     using C = SpecT<R>;
     if constexpr (plane_fft_fits<C, XN1, XN2, ZN1, ZN2>()) {
-        cudaError_t e = set((const void*)k_div_fft2<R, XN1, XN2, ZN1, ZN2>, bytes);
+        cudaError_t e = set((const void*)k_div_fft2<R, true, XN1, XN2, ZN1, ZN2>, bytes);
+        if constexpr (sizeof(R) == 8)
+            if (e == cudaSuccess) e = set((const void*)k_div_fft2<R, false, XN1, XN2, ZN1, ZN2>, bytes);
         if (e == cudaSuccess) e = set((const void*)k_fft2_inv<XN1, XN2, ZN1, ZN2, C>, bytes);
         return e;
     }
     return cudaErrorInvalidValue;
 }
-template <typename R, int XN1, int XN2, int ZN1, int ZN2>
+template <typename R, bool ST, int XN1, int XN2, int ZN1, int ZN2>
 void plane_fft_fwd(bool pdl, const Geo& g, const R* Q, R* RHSLL, SpecT<R>* SP, const DevState* st, int ns,
                    size_t smem, cudaStream_t s) {
     if constexpr (plane_fft_fits<SpecT<R>, XN1, XN2, ZN1, ZN2>())
-        launch_pdl(pdl, k_div_fft2<R, XN1, XN2, ZN1, ZN2>, g.M, (p2_nt<SpecT<R>, XN1 * XN2 * ZN1 * ZN2>()), smem, s, g, Q, RHSLL, SP, st, ns);
+        launch_pdl(pdl, k_div_fft2<R, ST, XN1, XN2, ZN1, ZN2>, g.M, (p2_nt<SpecT<R>, XN1 * XN2 * ZN1 * ZN2>()), smem, s, g, Q, RHSLL, SP, st, ns);
 }
 template <typename C, int XN1, int XN2, int ZN1, int ZN2>
 void plane_fft_inv(bool pdl, const Geo& g, const C* SP, typename CReal<C>::T* DPH, size_t smem, cudaStream_t s) {

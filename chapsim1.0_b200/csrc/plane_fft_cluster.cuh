@@ -8,7 +8,7 @@
 // transforms, twiddles, scalings and z-line pairing; only the division of the
 // work between blocks differs.
 //   k_div_fft2c  block r of the cluster of row j: DIVG_tg on the z lines
-//                k in [r NK, (r+1) NK) (NK = N / CS), written to RHSLLPHI;
+//                k in [r NK, (r+1) NK) (NK = N / CS), written to RHSLLPHI with ST;
 //                x transforms of their NK/2 packed pairs; unpacking of every
 //                kx and delivery of the two z values to the block that owns
 //                kx (kx in [r' KXC, (r'+1) KXC), KXC = ceil((L/2+1) / CS));
@@ -64,7 +64,7 @@ constexpr size_t p2c_smem() {
     return (size_t)P2cShape<NX1, NX2, NZ1, NZ2, CS>::WORDS * sizeof(C);
 }
 
-template <typename R, int NX1, int NX2, int NZ1, int NZ2, int CS>
+template <typename R, bool ST, int NX1, int NX2, int NZ1, int NZ2, int CS>
 __global__ void __launch_bounds__(p2c_nt<SpecT<R>>(), 1) k_div_fft2c(Geo g, const R* __restrict__ Q, R* __restrict__ RHSLL,
                                                          SpecT<R>* __restrict__ SP, const DevState* __restrict__ st,
                                                          int ns) {
@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(p2c_nt<SpecT<R>>(), 1) k_div_fft2c(Geo g, cons
                 out[e] = (R)x;
                 val[part][e] = (T)x;
             }
-            st16(RHSLL + iidx(g, i0, j, k), out);
+            if constexpr (ST) st16(RHSLL + iidx(g, i0, j, k), out);
         }
         C* line = xb + pair * LDX + i0;
 #pragma unroll
@@ -268,9 +268,10 @@ bool plane_fft_cluster_setup(const Geo& g) {
         return false;
     } else {
         constexpr size_t sm = p2c_smem<C, NX1, NX2, NZ1, NZ2, CS>();
-        auto kf = k_div_fft2c<R, NX1, NX2, NZ1, NZ2, CS>;
+        auto kf = k_div_fft2c<R, true, NX1, NX2, NZ1, NZ2, CS>;
+        auto kn = k_div_fft2c<R, sizeof(R) == 4, NX1, NX2, NZ1, NZ2, CS>;  // FP64: the form that stores no RHSLLPHI
         auto ki = k_fft2c_inv<NX1, NX2, NZ1, NZ2, CS, C>;
-        for (const void* k : {(const void*)kf, (const void*)ki}) {
+        for (const void* k : {(const void*)kf, (const void*)kn, (const void*)ki}) {
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess) return false;
             if (CS > 8 && cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
                 return false;
@@ -286,20 +287,21 @@ bool plane_fft_cluster_setup(const Geo& g) {
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        int nf = 0, ni = 0;
+        int nf = 0, nn = 0, ni = 0;
         if (cudaOccupancyMaxActiveClusters(&nf, kf, &cfg) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (cudaOccupancyMaxActiveClusters(&nn, kn, &cfg) != cudaSuccess) { cudaGetLastError(); return false; }
         if (cudaOccupancyMaxActiveClusters(&ni, ki, &cfg) != cudaSuccess) { cudaGetLastError(); return false; }
-        return nf > 0 && ni > 0;
+        return nf > 0 && nn > 0 && ni > 0;
     }
 }
 
-template <typename R, int NX1, int NX2, int NZ1, int NZ2>
+template <typename R, bool ST, int NX1, int NX2, int NZ1, int NZ2>
 void plane_fft_cluster_fwd(bool pdl, const Geo& g, const R* Q, R* RHSLL, SpecT<R>* SP, const DevState* st, int ns,
                            cudaStream_t s) {
     using C = SpecT<R>;
     constexpr int CS = p2c_cluster<C, NX1, NX2, NZ1, NZ2>();
     if constexpr (CS != 0)
-        launch_cluster(pdl, CS, k_div_fft2c<R, NX1, NX2, NZ1, NZ2, CS>, dim3(CS, g.M), dim3(p2c_nt<C>()),
+        launch_cluster(pdl, CS, k_div_fft2c<R, ST, NX1, NX2, NZ1, NZ2, CS>, dim3(CS, g.M), dim3(p2c_nt<C>()),
                        p2c_smem<C, NX1, NX2, NZ1, NZ2, CS>(), s, g, Q, RHSLL, SP, st, ns);
 }
 template <typename C, int NX1, int NX2, int NZ1, int NZ2>

@@ -6,7 +6,7 @@
 //   BC_WALL_PR_tg (src/BC_WALL.f90:293-361).
 //
 // Kernels:
-//   k_div_fftx   divergence of u* / (alpha dt) -> RHSLLPHI, then the real
+//   k_div_fftx   divergence of u* / (alpha dt) (-> RHSLLPHI where k_correct reads it), then the real
 //                x transform of every (j, k) line (two real lines packed in
 //                one complex FFT), times 1/L, into the spectral array
 //   k_fftz<S>    complex z transform of every (kx, j) line; forward pass
@@ -57,8 +57,8 @@ template <typename C> __host__ __device__ constexpr int px_minb() { return sizeo
 // ---------------------------------------------------------------------------
 // R is the stored type of Q, PR, RHSLLPHI and DPH (double, or float in the
 // mixed-precision step, whose x and z transforms also run in FP32); the
-// divergence and the correction are evaluated in FP64.
-template <typename R, int N1, int N2>
+// divergence and the correction are evaluated in FP64.  ST: RHSLLPHI is stored (see k_correct).
+template <typename R, bool ST, int N1, int N2>
 __global__ void __launch_bounds__(PX_NT, px_minb<SpecT<R>>()) k_div_fftx(Geo g, const R* __restrict__ Q, R* __restrict__ RHSLL,
                                                     SpecT<R>* __restrict__ SP, const DevState* __restrict__ st, int ns) {
     pdl_wait();
@@ -78,8 +78,8 @@ __global__ void __launch_bounds__(PX_NT, px_minb<SpecT<R>>()) k_div_fftx(Geo g, 
     const double coe1 = g.dxi / 1.0;
     // one item = VW consecutive points of both rows of a packed pair (M is a multiple of 32: every row of the
     // tile exists), read with 16-byte loads and no branch between them, so that all of two items' loads are in
-    // flight together: waits for them were 0.7 of the kernel's stalls at 2.5 TB/s.  Per step 1.42 -> 1.39 ms at
-    // 384 x 256 x 384, FP32 there 0.72 -> 0.59 ms (FP64 stores RHSLLPHI and loads twice the bytes).  The pair's complex
+    // flight together: waits for them were 0.7 of the kernel's stalls at 2.5 TB/s.  Per step 1.31 -> 1.13 ms at
+    // 384 x 256 x 384 (1.42 -> 1.39 with RHSLLPHI stored), 70 -> 56 us at 128^3, FP32 at 384 x 256 x 384 0.72 -> 0.59 ms.  The pair's complex
     // values are stored to shared memory together
     constexpr int VW = V16<R>::W, LV = L / VW, NI = NP * LV;
     auto item = [&](int p) {
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(PX_NT, px_minb<SpecT<R>>()) k_div_fftx(Geo g, 
                 out[e] = (R)x;
                 val[part][e] = (T)x;
             }
-            st16(RHSLL + iidx(g, i0, j + part, k), out);
+            if constexpr (ST) st16(RHSLL + iidx(g, i0, j + part, k), out);
         }
         C* line = smc + pair * LD + i0;
 #pragma unroll
@@ -1014,7 +1014,16 @@ __global__ void __launch_bounds__(px_nt<N1>(), (px_rminb<C, N1>())) k_fftx_inv(G
 // Each thread updates W = 16 / sizeof(R) consecutive points of an x line with
 // 16-byte loads and stores (L is a multiple of 4); the per-point arithmetic
 // is FP64, in the same order for every point.
-template <typename R>
+// PRCALC_tg subtracts BE times RHSLLPHI.  LAP (FP64, where lap_is_rhs of chapsim_gpu.cu finds that the caller's
+// operator is the discrete Laplacian, as the reference's is): the Laplacian of the Poisson solution stands for it
+// (AMPH, ACPH, APPH in y, second differences in x and z), from the DPH
+// neighbours that are in cache, so the divergence kernel need not write the array nor this one read it (two
+// words per point and substep).  The difference is the rounding of the Laplacian times BE = alpha dt nu / 2: relative
+// to DPH 2^-53 BE (4/dx^2 + 4/dz^2 + 4/dy^2), the diffusion number's size; over three fields PR differs from the oracle's
+// by 2.3e-16 rms where the array gives 2.0e-16 at REN = 2 (64 x 96 x 64, projection; 2.1e-16 with the sweeps and transforms
+// in shared memory), by the same 8.7e-16 at REN = 2800.  Divergence 1.39 -> 1.13 and
+// correction 1.45 -> 1.29 ms per step at 384 x 256 x 384, step 0.585 -> 0.567 ms at 128^3.  FP32 keeps the array.
+template <typename R, bool LAP>
 __global__ void __launch_bounds__(CR_NT) k_correct(Geo g, R* __restrict__ Q, R* __restrict__ PR,
                                                    const R* __restrict__ DPH, const R* __restrict__ RHSLL,
                                                    const DevState* __restrict__ st, int ns) {
@@ -1030,15 +1039,29 @@ __global__ void __launch_bounds__(CR_NT) k_correct(Geo g, R* __restrict__ Q, R* 
     const double dt = st->dt, ta = g.talp[ns];
     const long long c = pidx(g, i0, j, k);
     // all loads first: Q is read and written through one pointer
-    R ph[W], phk[W], phj[W], uu[W], vv[W], ww[W], pr[W], ll[W];
+    R ph[W], phk[W], phj[W], uu[W], vv[W], ww[W], pr[W], ll[W], phkp[W], phjp[W];
     ld16(DPH + c, ph);
     ld16(DPH + pidx(g, i0, j, wrapm(k, N)), phk);
     if (j >= 2) ld16(DPH + c - L, phj);
+    if constexpr (LAP) {
+        ld16(DPH + pidx(g, i0, j, wrapp(k, N)), phkp);
+        if (j < M) ld16(DPH + c + L, phjp);
+    }
     ld16(Q + c, uu);
     ld16(Q + c + g.FS, vv);
     ld16(Q + c + 2 * g.FS, ww);
     ld16(PR + c, pr);
-    ld16(RHSLL + iidx(g, i0, j, k), ll);
+    if constexpr (!LAP) ld16(RHSLL + iidx(g, i0, j, k), ll);
+    else {
+        const double phip0 = DPH[pidx(g, i0 + W == L ? 0 : i0 + W, j, k)], pl = DPH[pidx(g, wrapm(i0, L), j, k)];
+        const double am = j >= 2 ? g.amph[j] : 0.0, ap = j < M ? g.apph[j] : 0.0, ac = g.acph[j];
+#pragma unroll
+        for (int e = 0; e < W; ++e) {
+            const double p = ph[e], px = e == W - 1 ? phip0 : ph[e + 1 < W ? e + 1 : e], pm = e == 0 ? pl : ph[e > 0 ? e - 1 : e];
+            const double y = (j >= 2 ? am * phj[e] : 0.0) + ac * p + (j < M ? ap * phjp[e] : 0.0);
+            ll[e] = ((px - p) - (p - pm)) * g.dxqi + ((phkp[e] - p) - (p - phk[e])) * g.dzqi + y;
+        }
+    }
     const double phim0 = DPH[pidx(g, wrapm(i0, L), j, k)];
     const double cx = dt * ta * g.dxi, cz = dt * ta * g.dzi, cy = dt * ta * g.dyci[j] / 1.0;
     const double be = 0.5 * ta * dt * g.cvisc * 1.0 / 1.0;
