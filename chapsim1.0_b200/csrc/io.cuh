@@ -528,7 +528,10 @@ struct IoTileAcc {  // neighbours of one point in the tile's planes
         const double dx = (q(0, di + 1, dj, dk) - q(0, di, dj, dk)) * dxi;
         const double dy = (q(1, di, dj + 1, dk) - q(1, di, dj, dk)) * (dj < 0 ? dyfim : dyfij);
         const double dz = (q(2, di, dj, dk + 1) - q(2, di, dj, dk)) * dzi;
-        return (dx + dy + dz) * (1.0 / 3.0);
+        // the quotient by 3, correctly rounded as in DIVG_U_io: a product by the rounded reciprocal and its correction
+        // (Markstein, see io_cn.cuh); the product alone has 1.2 times the rounding error where div(u) is not small
+        const double sum = dx + dy + dz, q3 = sum * (1.0 / 3.0);
+        return fma(fma(-3.0, q3, sum), 1.0 / 3.0, q3);
     }
 };
 
