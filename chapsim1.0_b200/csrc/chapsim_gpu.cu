@@ -3212,12 +3212,13 @@ extern "C" int chapsim_batch_advance(chapsim_batch_t* b, int32_t nsteps, double 
     }
     cudaError_t e = cudaStreamSynchronize(b->stream);
     if (e != cudaSuccess) return fail(nullptr, CHAPSIM_ERR_CUDA, std::string("ensemble sync: ") + cudaGetErrorString(e));
+    int rc = CHAPSIM_OK;  // the first member's error; every member's word is read and cleared
     for (chapsim_ctx* c : b->ctx) {
         c->launches += (unsigned long long)nsteps * (unsigned long long)(b->kernels_per_step / (int)b->ctx.size());
-        int rc = check_device_error(c);
-        if (rc) return fail(nullptr, rc, c->err);
+        const int rc_c = check_device_error(c);
+        if (rc_c && !rc) rc = fail(nullptr, rc_c, c->err);
     }
-    return CHAPSIM_OK;
+    return rc;
 }
 
 extern "C" int chapsim_batch_get_stream(chapsim_batch_t* b, void** stream) {

@@ -46,6 +46,37 @@ def test_ensemble_follows_its_members_settings(force):
         c.close()
 
 
+def test_ensemble_error_is_not_carried_into_the_next_call():
+    """Two of three members report a NaN; with good fields in all of them the ensemble advances as new members do."""
+    shapes = [(32, 32, 32), (64, 32, 32), (32, 64, 32)]
+    out = []
+    for bad in (False, True):
+        grp = [_channel(sh, 91 + k) for k, sh in enumerate(shapes)]
+        e = gpu.Ensemble(grp)
+        if bad:
+            good = [c.download() for c in grp]
+            for c, (Q, PR) in zip(grp[::2], good[::2]):
+                Qn = Q.copy()
+                Qn[0, 3, 5, 7] = float("nan")
+                c.upload(Qn, PR)
+            with pytest.raises(gpu.ChapsimError) as err:
+                e.advance(1, 2e-3, 1e-6, 0.5)
+            assert err.value.code == -2
+            for c, (Q, PR) in zip(grp, good):
+                c.upload(Q, PR)
+                c.set_dt(2e-3)
+        else:
+            for c in grp:  # as the others, through the host
+                c.upload(*c.download())
+        e.advance(2, 2e-3, 1e-6, 0.5)
+        out.append([x for c in grp for x in c.download()])
+        e.close()
+        for c in grp:
+            c.close()
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
+
+
 def _heated(seed=63):
     L = M = N = 32
     s = channel_setup(L, M, N, 2 * math.pi, math.pi, 2.0, 2800.0)
