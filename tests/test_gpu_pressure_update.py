@@ -1,7 +1,7 @@
 """PRCALC_tg: PR + DPH - alpha dt nu / 2 RHSLLPHI, with RHSLLPHI the divergence that the Poisson solve was given.
 
 The FP64 update takes the discrete Laplacian of DPH for it, which holds for the reference's Poisson operator only: the
-caller's wavenumbers AK1 and AK3 need not be the second difference's, nor his rows AMPH, ACPH, APPH conservative with
+caller's wavenumbers AK1 and AK3 need not be the second difference's, nor the rows AMPH, ACPH, APPH conservative with
 Neumann walls.  With the exact second derivative's wavenumbers, and with an upper wall row of a fixed pressure, the FP64
 context is held to the mixed-precision one (which keeps RHSLLPHI) at REN = 2, where the term is of DPH's own size.  Bound:
 the FP32 velocities' rounding, 2^-24, enters RHSLLPHI times alpha dt nu / 2 as 2^-24 |u| nu 3 / dx < 1e-6 and DPH by less,
